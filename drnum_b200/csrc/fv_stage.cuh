@@ -9,14 +9,14 @@
 //     marches along i through a chunk of planes;
 //   - each plane of the stencil state is staged once in shared memory with a
 //     two-cell halo in j and k, in a ring of three planes (i .. i+2; the own
-//     column of plane i-1 is kept in registers); plane i+2 is loaded while
+//     column of plane i-1 is set aside beside it); plane i+2 is loaded while
 //     the y and z faces of plane i are evaluated: by one TMA box load where
 //     no periodic seam crosses the tile's halo, else cell by cell with
 //     cp.async;
-//   - every face flux is evaluated exactly once: x faces per thread along its
-//     own column (the upper face of cell i is kept in registers as the lower
-//     face of cell i+1), y and z faces of the current plane into shared
-//     memory;
+//   - every face flux is evaluated exactly once (fv_f64.cuh): x faces per
+//     thread along its own column (the upper face of cell i is kept in
+//     registers as the lower face of cell i+1), y and z faces of the current
+//     plane into shared memory;
 //   - the residual is summed per cell in registers in the reference's order
 //     (+Fx_lo +Fy_lo +Fz_lo -Fz_hi -Fy_hi -Fx_hi, the order the single-thread
 //     CPU iterator produces, cartesianiterator.h:115-188), no atomics;
@@ -33,6 +33,7 @@
 
 #include <cstdint>
 #include "fv_numerics.cuh"
+#include "fv_f64.cuh"
 #include "fv_wall.cuh"
 #include "fv_tma.cuh"
 
@@ -60,11 +61,12 @@ struct StageArgs {
 // index along an axis with periodic wrap; returns -1 if outside a closed axis
 __device__ __forceinline__ int axis_idx(int x, int n, int per)
 {
-  if (per) {
-    x %= n;
-    return x < 0 ? x + n : x;
-  }
-  return (x < 0 || x >= n) ? -1 : x;
+  if ((unsigned)x < (unsigned)n) return x;
+  if (!per) return -1;
+  x = x < 0 ? x + n : x - n;                     // one wrap, but for tiles reaching far beyond a small patch
+  if ((unsigned)x < (unsigned)n) return x;
+  x %= n;
+  return x < 0 ? x + n : x;
 }
 
 // does the face below cell index x (between x-1 and x) exist?
@@ -86,80 +88,36 @@ struct StageSmem {
   using FaceT = typename Policy::FaceT;
   static constexpr int PJ = TJ + 4;
   static constexpr int PK = TK + 4;
-  alignas(128) Real plane[3][5][PJ][PK];   // planes i .. i+2 (plane i-1 of the own column is kept in registers)
+  alignas(128) Real plane[3][5][PJ][PK];   // planes i .. i+2
+  Real xm[5][TJ * TK];                     // own column of plane i-1 (each thread its own cell)
   FaceT fy[5][TJ + 1][TK];
   FaceT fz[5][TJ][TK + 1];
   alignas(8) uint64_t bar;                 // mbarrier of the TMA plane loads
 };
 
-// Plane ip into ring slot `slot` cell by cell: cp.async of the cells inside
-// the patch (wrapped on periodic axes), zero for cells outside a closed one
-// (never read).  The caller commits and waits.
-template <class Policy, int TJ, int TK>
-__device__ __forceinline__ void load_plane_async(StageSmem<Policy, TJ, TK>& sm, int slot,
-                                                 const typename Policy::Store* __restrict__ in,
-                                                 const StageGeom& g, int i, int j0, int k0)
-{
-  static_assert(sizeof(typename Policy::Store) == 8 && sizeof(typename Policy::Real) == 8,
-                "cell copies move the stored 8-byte value unchanged");
-  constexpr int PJ = TJ + 4, PK = TK + 4;
-  const size_t nc = (size_t)g.ni * g.nj * g.nk;
-  const int tid = threadIdx.y * TK + threadIdx.x;
-  for (int e = tid; e < 5 * PJ * PK; e += TJ * TK) {
-    const int v = e / (PJ * PK);
-    const int rem = e - v * (PJ * PK);
-    const int jj = rem / PK;
-    const int kk = rem - jj * PK;
-    const int j = axis_idx(j0 - 2 + jj, g.nj, g.per_y);
-    const int k = axis_idx(k0 - 2 + kk, g.nk, g.per_z);
-    typename Policy::Real* dst = &sm.plane[slot][v][jj][kk];
-    if (j >= 0 && k >= 0) {
-      const unsigned sa = smem_u32(dst);
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;"
-                   :: "r"(sa), "l"(in + v * nc + ((size_t)i * g.nj + j) * g.nk + k) : "memory");
-    } else {
-      *dst = typename Policy::Real(0);
-    }
-  }
-  asm volatile("cp.async.commit_group;" ::: "memory");
-}
-
-template <class Policy, int TJ, int TK>
-__device__ __forceinline__ void load_plane(StageSmem<Policy, TJ, TK>& sm, int slot,
-                                           const typename Policy::Store* __restrict__ in,
-                                           const typename Policy::Params& pp,
-                                           const StageGeom& g, int ip, int j0, int k0)
-{
-  using Real = typename Policy::Real;
-  constexpr int PJ = TJ + 4, PK = TK + 4;
-  const int i = axis_idx(ip, g.ni, g.per_x);
-  if (i < 0) return;                      // plane outside a closed patch: never read
-  const size_t nc = (size_t)g.ni * g.nj * g.nk;
-  const int tid = threadIdx.y * TK + threadIdx.x;
-  for (int e = tid; e < 5 * PJ * PK; e += TJ * TK) {
-    const int v = e / (PJ * PK);
-    const int rem = e - v * (PJ * PK);
-    const int jj = rem / PK;
-    const int kk = rem - jj * PK;
-    const int j = axis_idx(j0 - 2 + jj, g.nj, g.per_y);
-    const int k = axis_idx(k0 - 2 + kk, g.nk, g.per_z);
-    Real val = Real(0);
-    if (j >= 0 && k >= 0) {
-      val = Policy::load(pp, v, in[v * nc + ((size_t)i * g.nj + j) * g.nk + k]);
-    }
-    sm.plane[slot][v][jj][kk] = val;
-  }
-}
+// Resident CTAs per SM the register allocation is sized for: 16 warps of 128
+// registers (the unconstrained 138 cost a quarter of the warps).
+template <int NT>
+struct F64Occupancy {
+  static constexpr int min_blocks = NT >= 512 ? 1 : 512 / NT;
+};
 
 // One tile of one patch: columns (j0 .. j0+TJ-1, k0 .. k0+TK-1), planes i0 .. i1-1.
 // tm: tensor map of the stage input with box (TK+4, TJ+4, 1, 5), or null.
-template <class Policy, int TJ, int TK>
+//
+// A plane's faces run through one copy of the face code (per thread its y, z
+// and x face, two warps one halo face more): four inlined copies, one per
+// use, overflowed the instruction cache.
+template <class Policy, class Scheme, int TJ, int TK>
 __device__ __forceinline__ void fv_stage_tile(const StageArgs<Policy>& a, const CUtensorMap* tm, int j0, int k0,
                                               int i0, int i1)
 {
   using Real = typename Policy::Real;
-  using FaceT = typename Policy::FaceT;
   using Smem = StageSmem<Policy, TJ, TK>;
+  static_assert(sizeof(typename Policy::Store) == 8 && sizeof(Real) == 8, "cell copies move the stored 8-byte value");
+  constexpr int PJ = TJ + 4, PK = TK + 4, NT = TJ * TK, NW = NT / 32;
+  constexpr int VS = PJ * PK, SS = 5 * VS;          // variable and slot strides of the ring
+  constexpr int PPT = (VS + NT - 1) / NT;           // positions of a plane per thread and variable
   extern __shared__ __align__(128) unsigned char dn_smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(dn_smem_raw);
 
@@ -168,15 +126,18 @@ __device__ __forceinline__ void fv_stage_tile(const StageArgs<Policy>& a, const 
   const int j = j0 + ty, k = k0 + tx;
   const bool own = (j < g.nj) && (k < g.nk);
   const size_t nc = (size_t)g.ni * g.nj * g.nk;
-  const Real Ax = a.p.Ax, Ay = a.p.Ay, Az = a.p.Az;
+  const size_t njk = (size_t)g.nj * g.nk;
   const int tid = ty * TK + tx;
+  const int warp = tid >> 5, lane = tid & 31;
+  Real* const ring = &sm.plane[0][0][0][0];
+  const int me = (ty + 2) * PK + tx + 2;            // own cell in a plane of the ring
   // TMA plane loads where no periodic seam crosses the tile's halo (on a
   // closed axis the box cells outside the patch are zero-filled, as the
   // cell copies write them); the box starts at column k0-2, a multiple of 2
   // elements (16 bytes) since TK is even
-  constexpr unsigned kPlaneBytes = 5u * (TJ + 4) * (TK + 4) * sizeof(Real);
+  constexpr unsigned kPlaneBytes = 5u * VS * sizeof(Real);
   const bool tma = tm != nullptr && (!g.per_y || (j0 >= 2 && j0 + TJ + 2 <= g.nj)) &&
-                   (!g.per_z || (k0 >= 2 && k0 + TK + 2 <= g.nk)) && (smem_u32(&sm.plane[0][0][0][0]) & 127) == 0;
+                   (!g.per_z || (k0 >= 2 && k0 + TK + 2 <= g.nk)) && (smem_u32(ring) & 127) == 0;
   if (tma && tid == 0) {
     mbar_init(&sm.bar, 1);
     mbar_init_fence();
@@ -184,212 +145,206 @@ __device__ __forceinline__ void fv_stage_tile(const StageArgs<Policy>& a, const 
   unsigned phase = 0;
   bool tbad = false;
 
-  // a three-plane ring, slot of plane p = p mod 3, rotated by hand: sa, sb,
-  // sc hold planes i-1, i, i+1 at the top of iteration i
-  int sa = (i0 + 2) % 3, sb = i0 % 3, sc = (i0 + 1) % 3;
-  // prologue: planes i0-1 .. i0+1 and the x face below cell i0; the own
-  // column of plane i0-2 comes straight from memory
-  for (int q = -1; q <= 1; ++q) load_plane<Policy, TJ, TK>(sm, (i0 + q + 3) % 3, a.in, a.p, g, i0 + q, j0, k0);
+  // in-plane offsets of this thread's positions for cell copies (-1: outside a closed axis)
+  int poff[PPT];
+  #pragma unroll
+  for (int m = 0; m < PPT; ++m) {
+    const int e = tid + m * NT;
+    const int jg = axis_idx(j0 - 2 + e / PK, g.nj, g.per_y), kg = axis_idx(k0 - 2 + e % PK, g.nk, g.per_z);
+    poff[m] = (e < VS && jg >= 0 && kg >= 0) ? jg * g.nk + kg : -1;
+  }
+  // plane i (inside the patch) into ring slot `slot` cell by cell: cp.async
+  // of the cells inside the patch, zero outside a closed axis (never read)
+  auto copy_plane = [&](int slot, int i) {
+    const Real* src = a.in + (size_t)i * njk;
+    Real* dst = ring + slot * SS;
+    #pragma unroll
+    for (int m = 0; m < PPT; ++m) {
+      const int e = tid + m * NT;
+      if (e >= VS) continue;
+      #pragma unroll
+      for (int v = 0; v < 5; ++v) {
+        if (poff[m] >= 0) {
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;"
+                       :: "r"(smem_u32(dst + v * VS + e)), "l"(src + v * nc + poff[m]) : "memory");
+        } else {
+          dst[v * VS + e] = Real(0);
+        }
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  // a three-plane ring, rotated by hand: sa, sb, sc hold planes i-1, i, i+1
+  // at the top of iteration i.  Prologue: planes i0-1 .. i0+1, and the own
+  // column of plane i0-2 (plane i0-1 again where it does not exist)
+  int sa = 0, sb = 1, sc = 2;
+  for (int q = -1; q <= 1; ++q) {
+    const int ip = axis_idx(i0 + q, g.ni, g.per_x);
+    if (ip >= 0) copy_plane(q + 1, ip);   // planes outside a closed patch are never read
+  }
+  const bool face0 = face_exists(i0, g.ni, g.per_x);
+  if (own && face0) {
+    const Real* col = a.in + (size_t)axis_idx(cell_ok(i0 - 2, g.ni, g.per_x) ? i0 - 2 : i0 - 1, g.ni, g.per_x) * njk +
+                      (size_t)j * g.nk + k;
+    #pragma unroll
+    for (int v = 0; v < 5; ++v) sm.xm[v][tid] = col[v * nc];
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
 
-  FaceT fx_lo[5];
-  {
-    const bool ex = face_exists(i0, g.ni, g.per_x);
-    if (ex && own) {
-      Real vl[5], vr[5], F[5];
-      const bool sl = cell_ok(i0 - 2, g.ni, g.per_x);
-      const bool sr = cell_ok(i0 + 1, g.ni, g.per_x);
-      const int im2 = axis_idx(i0 - 2, g.ni, g.per_x);
-      #pragma unroll
-      for (int v = 0; v < 5; ++v) {
-        const Real um2 = sl ? Policy::load(a.p, v, a.in[v * nc + ((size_t)im2 * g.nj + j) * g.nk + k]) : Real(0);
-        const Real um1 = sm.plane[sa][v][ty + 2][tx + 2];
-        const Real up0 = sm.plane[sb][v][ty + 2][tx + 2];
-        const Real up1 = sm.plane[sc][v][ty + 2][tx + 2];
-        vl[v] = upwind2_left(um2, um1, up0, sl);
-        vr[v] = upwind2_right(um1, up0, up1, sr);
-      }
-      ausm_plus<0>(face_side(vl), face_side(vr), Ax, F);
-      #pragma unroll
-      for (int v = 0; v < 5; ++v) fx_lo[v] = Policy::face(a.p, v, F[v]);
+  const bool ey = face_exists(j, g.nj, g.per_y) && k < g.nk && (g.per_y || j < g.nj);
+  const bool ez = face_exists(k, g.nk, g.per_z) && j < g.nj && (g.per_z || k < g.nk);
+  Real fx_lo[5];
+  // iteration i0-1 evaluates the x face below cell i0 only
+  for (int i = i0 - 1; i < i1; ++i) {
+    const bool first = i < i0;
+    int s0, sp1, sp2;                     // slots of planes i, i+1, i+2
+    int ip2 = -1;
+    if (first) {
+      s0 = sa; sp1 = sb; sp2 = sc;
     } else {
+      // plane i+2 replaces plane i-1 in the ring; the own column of plane
+      // i-1 (the x face above cell i reads it) is set aside first (plane i
+      // itself where plane i-1 lies outside a closed patch)
+      const Real* src = ring + (cell_ok(i - 1, g.ni, g.per_x) ? sa : sb) * SS + me;
       #pragma unroll
-      for (int v = 0; v < 5; ++v) fx_lo[v] = FaceT(0);
-    }
-  }
-
-  for (int i = i0; i < i1; ++i) {
-    // plane i+2 replaces plane i-1 in the ring; the own column of plane i-1
-    // (the x face above cell i reads it) moves to registers first
-    Real xm1[5];
-    #pragma unroll
-    for (int v = 0; v < 5; ++v) xm1[v] = sm.plane[sa][v][ty + 2][tx + 2];
-    __syncthreads();
-    // plane i+2 into the freed slot, arriving while the y and z faces of
-    // plane i are evaluated (a plane outside a closed patch is never read)
-    const int ip2 = axis_idx(i + 2, g.ni, g.per_x);
-    if (ip2 >= 0) {
-      if (tma) {
-        if (tid == 0) {
-          fence_proxy_async_smem();
-          mbar_arrive_expect_tx(&sm.bar, kPlaneBytes);
-          tma_load_4d(&sm.plane[sa][0][0][0], tm, &sm.bar, k0 - 2, j0 - 2, ip2, 0);
+      for (int v = 0; v < 5; ++v) sm.xm[v][tid] = src[v * VS];
+      __syncthreads();
+      // plane i+2 into the freed slot, arriving while the y and z faces of
+      // plane i are evaluated (a plane outside a closed patch is never read)
+      ip2 = axis_idx(i + 2, g.ni, g.per_x);
+      if (ip2 >= 0) {
+        if (tma) {
+          if (tid == 0) {
+            fence_proxy_async_smem();
+            mbar_arrive_expect_tx(&sm.bar, kPlaneBytes);
+            tma_load_4d(ring + sa * SS, tm, &sm.bar, k0 - 2, j0 - 2, ip2, 0);
+          }
+        } else {
+          copy_plane(sa, ip2);
         }
-      } else {
-        load_plane_async<Policy, TJ, TK>(sm, sa, a.in, g, ip2, j0, k0);
       }
+      s0 = sb; sp1 = sc; sp2 = sa;
     }
-    const int s0 = sb, sp1 = sc, sp2 = sa;
 
-    // y faces of plane i: face at row jj (0..TJ) lies below cell j0+jj
-    // (the items beyond one per thread, the faces below halo row TJ, fall to
-    // the last warp, and those of the z loop below to the one before it, so
-    // that no warp evaluates more than one extra face per plane)
-    for (int f = (ty * TK + tx + 32) % (TJ * TK); f < (TJ + 1) * TK; f += TJ * TK) {
-      const int jj = f / TK, kk = f - jj * TK;
-      const int jf = j0 + jj, kf = k0 + kk;
-      FaceT out[5];
-      const bool ex = face_exists(jf, g.nj, g.per_y) && kf < g.nk && (g.per_y || jf < g.nj);
+    Real F[5];
+    #pragma unroll 1
+    for (int t = first ? 3 : 0; t < 4; ++t) {
+      // t = 0, 1: the y and z faces below the own cell; 2: the faces below
+      // halo row TJ (last warp) and halo column TK (the warp before it); 3:
+      // the x face above the own cell
+      if (t == 2 && warp < NW - 2) continue;
+      FaceCells c;
+      int dir;
+      bool ex;
+      Real A;
+      Real* o = nullptr;
+      int os = 0;
+      if (t == 3) {
+        if (!first) {
+          // plane i+2 has arrived (this thread's copies, or the TMA box);
+          // the barrier publishes it and the y and z faces
+          if (ip2 >= 0) {
+            if (tma) {
+              tbad |= !mbar_wait(&sm.bar, phase);
+              phase ^= 1u;
+            } else {
+              asm volatile("cp.async.wait_group 0;" ::: "memory");
+            }
+          }
+          __syncthreads();
+        }
+        dir = 0;
+        A = a.p.Ax;
+        ex = own && face_exists(i + 1, g.ni, g.per_x);
+        c.sl = cell_ok(i - 1, g.ni, g.per_x);
+        c.sr = cell_ok(i + 2, g.ni, g.per_x);
+        c.m2 = &sm.xm[0][tid];
+        c.s2 = NT;
+        c.m1 = ring + s0 * SS + me;
+        c.p0 = ring + sp1 * SS + me;
+        c.p1 = ring + (c.sr ? sp2 : sp1) * SS + me;
+      } else {
+        const bool halo = t == 2;
+        dir = halo ? (warp == NW - 1 ? 1 : 2) : t + 1;
+        const bool ydir = dir == 1;
+        const int jj = halo ? (ydir ? TJ : lane) : ty, kk = halo ? (ydir ? lane : TK) : tx;
+        const int jf = j0 + jj, kf = k0 + kk;
+        if (ydir) {
+          ex = halo ? (lane < TK && face_exists(jf, g.nj, g.per_y) && kf < g.nk && (g.per_y || jf < g.nj)) : ey;
+          c.sl = cell_ok(jf - 2, g.nj, g.per_y);
+          c.sr = cell_ok(jf + 1, g.nj, g.per_y);
+          A = a.p.Ay;
+          if (!halo || lane < TK) o = &sm.fy[0][jj][kk];
+          os = (TJ + 1) * TK;
+        } else {
+          ex = halo ? (lane < TJ && face_exists(kf, g.nk, g.per_z) && jf < g.nj && (g.per_z || kf < g.nk)) : ez;
+          c.sl = cell_ok(kf - 2, g.nk, g.per_z);
+          c.sr = cell_ok(kf + 1, g.nk, g.per_z);
+          A = a.p.Az;
+          if (!halo || lane < TJ) o = &sm.fz[0][jj][kk];
+          os = TJ * (TK + 1);
+        }
+        const int step = ydir ? PK : 1;
+        c.p0 = ring + s0 * SS + (jj + 2) * PK + kk + 2;
+        c.m1 = c.p0 - step;
+        c.m2 = c.m1 - (c.sl ? step : 0);
+        c.p1 = c.p0 + (c.sr ? step : 0);
+        c.s2 = VS;
+      }
       if (ex) {
-        Real vl[5], vr[5], F[5];
-        const bool sl = cell_ok(jf - 2, g.nj, g.per_y);
-        const bool sr = cell_ok(jf + 1, g.nj, g.per_y);
-        #pragma unroll
-        for (int v = 0; v < 5; ++v) {
-          const Real um2 = sm.plane[s0][v][jj][kk + 2];
-          const Real um1 = sm.plane[s0][v][jj + 1][kk + 2];
-          const Real up0 = sm.plane[s0][v][jj + 2][kk + 2];
-          const Real up1 = sm.plane[s0][v][jj + 3][kk + 2];
-          vl[v] = upwind2_left(um2, um1, up0, sl);
-          vr[v] = upwind2_right(um1, up0, up1, sr);
-        }
-        ausm_plus<1>(face_side(vl), face_side(vr), Ay, F);
-        #pragma unroll
-        for (int v = 0; v < 5; ++v) out[v] = Policy::face(a.p, v, F[v]);
+        face_flux<Scheme, VS>(dir, c, A, F);
       } else {
         #pragma unroll
-        for (int v = 0; v < 5; ++v) out[v] = FaceT(0);
+        for (int v = 0; v < 5; ++v) F[v] = Real(0);
       }
-      #pragma unroll
-      for (int v = 0; v < 5; ++v) sm.fy[v][jj][kk] = out[v];
-    }
-
-    // z faces of plane i: face at column kk (0..TK) lies below cell k0+kk
-    for (int f = (ty * TK + tx + 64) % (TJ * TK); f < TJ * (TK + 1); f += TJ * TK) {
-      const int jj = f / (TK + 1), kk = f - jj * (TK + 1);
-      const int jf = j0 + jj, kf = k0 + kk;
-      FaceT out[5];
-      const bool ex = face_exists(kf, g.nk, g.per_z) && jf < g.nj && (g.per_z || kf < g.nk);
-      if (ex) {
-        Real vl[5], vr[5], F[5];
-        const bool sl = cell_ok(kf - 2, g.nk, g.per_z);
-        const bool sr = cell_ok(kf + 1, g.nk, g.per_z);
+      if (o) {
         #pragma unroll
-        for (int v = 0; v < 5; ++v) {
-          const Real um2 = sm.plane[s0][v][jj + 2][kk];
-          const Real um1 = sm.plane[s0][v][jj + 2][kk + 1];
-          const Real up0 = sm.plane[s0][v][jj + 2][kk + 2];
-          const Real up1 = sm.plane[s0][v][jj + 2][kk + 3];
-          vl[v] = upwind2_left(um2, um1, up0, sl);
-          vr[v] = upwind2_right(um1, up0, up1, sr);
-        }
-        ausm_plus<2>(face_side(vl), face_side(vr), Az, F);
-        #pragma unroll
-        for (int v = 0; v < 5; ++v) out[v] = Policy::face(a.p, v, F[v]);
-      } else {
-        #pragma unroll
-        for (int v = 0; v < 5; ++v) out[v] = FaceT(0);
-      }
-      #pragma unroll
-      for (int v = 0; v < 5; ++v) sm.fz[v][jj][kk] = out[v];
-    }
-    // plane i+2 has arrived (this thread's copies, or the TMA box); the
-    // barrier publishes it and the y and z faces
-    if (ip2 >= 0) {
-      if (tma) {
-        tbad |= !mbar_wait(&sm.bar, phase);
-        phase ^= 1u;
-      } else {
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-      }
-    }
-    __syncthreads();
-
-    // x face above cell i (between i and i+1), own column
-    FaceT fx_hi[5];
-    {
-
-      const bool ex = face_exists(i + 1, g.ni, g.per_x);
-      if (ex && own) {
-        Real vl[5], vr[5], F[5];
-        const bool sl = cell_ok(i - 1, g.ni, g.per_x);
-        const bool sr = cell_ok(i + 2, g.ni, g.per_x);
-        #pragma unroll
-        for (int v = 0; v < 5; ++v) {
-          const Real um2 = xm1[v];
-          const Real um1 = sm.plane[s0][v][ty + 2][tx + 2];
-          const Real up0 = sm.plane[sp1][v][ty + 2][tx + 2];
-          const Real up1 = sm.plane[sp2][v][ty + 2][tx + 2];
-          vl[v] = upwind2_left(um2, um1, up0, sl);
-          vr[v] = upwind2_right(um1, up0, up1, sr);
-        }
-        ausm_plus<0>(face_side(vl), face_side(vr), Ax, F);
-        #pragma unroll
-        for (int v = 0; v < 5; ++v) fx_hi[v] = Policy::face(a.p, v, F[v]);
-      } else {
-        #pragma unroll
-        for (int v = 0; v < 5; ++v) fx_hi[v] = FaceT(0);
+        for (int v = 0; v < 5; ++v) o[v * os] = F[v];
       }
     }
 
-
-    if (own) {
-      const size_t c = ((size_t)i * g.nj + j) * g.nk + k;
+    if (!first && own) {
+      const size_t c = (size_t)i * njk + (size_t)j * g.nk + k;
       const bool act = a.active ? (a.active[c] != 0) : true;
       int bad = 0;
-      FaceT res[5];
+      Real res[5];
       #pragma unroll
       for (int v = 0; v < 5; ++v) {
-        FaceT r = fx_lo[v];
+        Real r = fx_lo[v];
         r += sm.fy[v][ty][tx];
         r += sm.fz[v][ty][tx];
         r -= sm.fz[v][ty][tx + 1];
         r -= sm.fy[v][ty + 1][tx];
-        r -= fx_hi[v];
+        r -= F[v];
         res[v] = r;
       }
       if (a.wall.any && (i == 0 || i == g.ni - 1 || j == 0 || j == g.nj - 1 || k == 0 || k == g.nk - 1)) {
         Real U[5];
         #pragma unroll
-        for (int v = 0; v < 5; ++v) U[v] = sm.plane[s0][v][ty + 2][tx + 2];
-        add_wall_fluxes(a.wall, g.ni, g.nj, g.nk, g.per_x, g.per_y, g.per_z, i, j, k, U, Ax, Ay, Az, res,
-                        [&](int v, Real F) { return Policy::face(a.p, v, F); });
+        for (int v = 0; v < 5; ++v) U[v] = ring[s0 * SS + v * VS + me];
+        add_wall_fluxes(a.wall, g.ni, g.nj, g.nk, g.per_x, g.per_y, g.per_z, i, j, k, U, a.p.Ax, a.p.Ay, a.p.Az, res,
+                        [&](int v, Real x) { return Policy::face(a.p, v, x); });
       }
       #pragma unroll
       for (int v = 0; v < 5; ++v) {
-        const int bad_before = bad;
-        const FaceT r = res[v];
         typename Policy::Store o;
         if (act) {
-          o = Policy::update(a.p, v, a.un[v * nc + c], r, bad);
+          o = Policy::update(a.p, v, a.un[v * nc + c], res[v], bad);
         } else {
           o = a.in[v * nc + c];
         }
         a.out[v * nc + c] = o;
-        if (bad != bad_before && a.err_info &&
-            atomicCAS(&a.err_info[0], ~0ull, (unsigned long long)c) == ~0ull) {
-          a.err_info[1] = (unsigned long long)v;
-          a.err_info[2] = (unsigned long long)__double_as_longlong((double)a.un[v * nc + c]);
-          a.err_info[3] = (unsigned long long)__double_as_longlong((double)r);
-        }
       }
-      if (bad && a.err) atomicOr(a.err, bad);
     }
     #pragma unroll
-    for (int v = 0; v < 5; ++v) fx_lo[v] = fx_hi[v];
-    sa = sb;
-    sb = sc;
-    sc = sp2;
+    for (int v = 0; v < 5; ++v) fx_lo[v] = F[v];
+    if (!first) {
+      sa = s0;
+      sb = sp1;
+      sc = sp2;
+    }
   }
   if (tbad && a.err) atomicOr(a.err, 32);
 }
@@ -405,11 +360,11 @@ struct StageLaunch {
 
 // One patch per launch: grid (k tiles, j tiles, i chunks).
 template <class Policy, int TJ, int TK>
-__global__ void __launch_bounds__(TJ * TK)
+__global__ void __launch_bounds__(TJ * TK, F64Occupancy<TJ * TK>::min_blocks)
 fv_stage_kernel(const __grid_constant__ StageLaunch<Policy> L)
 {
   const int i0 = blockIdx.z * L.a.g.i_chunk;
-  fv_stage_tile<Policy, TJ, TK>(L.a, L.tma ? &L.tm : nullptr, blockIdx.y * TJ, blockIdx.x * TK, i0,
+  fv_stage_tile<Policy, AusmPlusFace, TJ, TK>(L.a, L.tma ? &L.tm : nullptr, blockIdx.y * TJ, blockIdx.x * TK, i0,
                                 min(L.a.g.ni, i0 + L.a.g.i_chunk));
 }
 
