@@ -1401,6 +1401,12 @@ int build_batch(dn_ctx* c)
 
 int stage_patch(dn_ctx* c, DnPatch& p, int in_b, int un_b, int out_b, double factor);
 
+// Does a stage run as a functor of the generic stage (per patch)?
+bool functor_stage(const dn_ctx* c)
+{
+  return c->precision == DN_FP64 && (c->stage_fn || c->scheme == DN_FLUX_AUSMPLUS_FUNCTOR);
+}
+
 // An inactive (or unlisted) patch's state carried from buffer in_b into out_b.
 int carry_patch(dn_ctx* c, DnPatch& p, int in_b, int out_b)
 {
@@ -1422,8 +1428,8 @@ int stage_all(dn_ctx* c, int in_b, int un_b, int out_b, double factor)
   }
   // a single patch keeps its parameters in the kernel's constant bank (the
   // batched form reads them from shared memory); the results are identical.
-  // Flux functors (another scheme or a user stage function) run per patch.
-  const bool functor = c->precision == DN_FP64 && (c->scheme != DN_FLUX_AUSMPLUS || c->stage_fn);
+  // Flux functors (the generic stage or a user stage function) run per patch.
+  const bool functor = functor_stage(c);
   if (!c->batched || c->patches.size() == 1 || functor) {
     for (auto& p : c->patches) {
       if (!p.owned || !p.patch_active) continue;
@@ -1470,7 +1476,7 @@ int stage_all(dn_ctx* c, int in_b, int un_b, int out_b, double factor)
       b.factor = factor;
       b.err = c->d_err;
       b.err_info = c->d_err_info;
-      e = c->precision == DN_FP64 ? dn::launch_stage_f64_batched(b, q, st)
+      e = c->precision == DN_FP64 ? dn::launch_stage_f64_batched(b, c->scheme, q, st)
                                   : dn::launch_stage_fx32_batched(b, q, f, st);
       c->launches++;
       if (e != cudaSuccess) return cuda_fail(c, e, "batched stage launch");
@@ -1495,7 +1501,7 @@ int stage_patch(dn_ctx* c, DnPatch& p, int in_b, int un_b, int out_b, double fac
   g.per_y = p.d.face[1] == DN_FACE_PERIODIC;
   g.per_z = p.d.face[2] == DN_FACE_PERIODIC;
   cudaError_t e;
-  if (c->precision == DN_FP64 && (c->scheme != DN_FLUX_AUSMPLUS || c->stage_fn)) {
+  if (functor_stage(c)) {
     dn_stage_launch L;
     L.patch = (int)(&p - c->patches.data());
     L.in = (const double*)p.buf[in_b];
@@ -1514,7 +1520,7 @@ int stage_patch(dn_ctx* c, DnPatch& p, int in_b, int un_b, int out_b, double fac
       if (rc) return fail(c, rc < 0 ? rc : DN_ERR_ARG, "user stage function returned %d for patch %d", rc, L.patch);
       return DN_OK;
     }
-    e = dn::launch_scheme_stage(c->scheme, &L, p.wall);
+    e = dn::launch_ausm_functor_stage(&L, p.wall);
     if (e != cudaSuccess) return cuda_fail(c, e, "functor stage launch");
     return DN_OK;
   } else if (c->precision == DN_FP64) {
@@ -1529,7 +1535,7 @@ int stage_patch(dn_ctx* c, DnPatch& p, int in_b, int un_b, int out_b, double fac
     a.g = g;
     a.p.Ax = dy * dz; a.p.Ay = dx * dz; a.p.Az = dx * dy; a.p.pf = pf;
     a.wall = p.wall;
-    e = dn::launch_stage_f64(a, dn::StageShape{4, 32, g.i_chunk}, c->stream);
+    e = dn::launch_stage_f64(a, c->scheme, c->stream);
   } else {
     dn::FxArgs a;
     a.in = (const int32_t*)p.buf[in_b];

@@ -147,7 +147,7 @@ fx_stage_batched_persistent(const Batch b)
   }
 }
 
-template <int TJ, int TK>
+template <class Scheme, int TJ, int TK>
 __global__ void __launch_bounds__(TJ * TK, F64Occupancy<TJ * TK>::min_blocks)
 fv_stage_batched_f64(const Batch b)
 {
@@ -174,7 +174,7 @@ fv_stage_batched_f64(const Batch b)
   }
   __syncthreads();
   const BatchMaps* M = (b.maps && rec.tma) ? b.maps + w.patch : nullptr;
-  fv_stage_tile<PolicyF64, AusmPlusFace, TJ, TK>(args, M ? &M->in[b.in_b][0] : nullptr, w.j0, w.k0, w.i0, w.i1);
+  fv_stage_tile<PolicyF64, Scheme, TJ, TK>(args, M ? &M->in[b.in_b][0] : nullptr, w.j0, w.k0, w.i0, w.i1);
 }
 
 } // namespace dn

@@ -10,13 +10,8 @@
 
 namespace dn {
 
-// Tile and chunk shape of one launch.
-struct StageShape {
-  int tj, tk;      // CTA tile in j and k (threads = tj*tk)
-  int i_chunk;     // planes per CTA along i
-};
-
-cudaError_t launch_stage_f64(const StageArgs<PolicyF64>& a, const StageShape& s, cudaStream_t st);
+// scheme: DN_FLUX_AUSMPLUS, DN_FLUX_VANLEER or DN_FLUX_ROE
+cudaError_t launch_stage_f64(const StageArgs<PolicyF64>& a, int scheme, cudaStream_t st);
 // Tensor map of an FP64 stage input for tj x tk tiles (box tk+4 x tj+4 x 1 x
 // 5); false when the patch does not allow it (rows not 16-byte strided,
 // unaligned field) or DN_FX_NO_TMA=1 is set.
@@ -43,7 +38,7 @@ constexpr int kNumShapes = 3;
 cudaError_t launch_stage_fx32_batched(const Batch& b, int shape, int form, cudaStream_t st);
 // resident CTAs per SM of the batched FX32 kernel of a tile shape and form
 cudaError_t fx32_batched_occupancy(int shape, int form, int* blocks);
-cudaError_t launch_stage_f64_batched(const Batch& b, int shape, cudaStream_t st);
+cudaError_t launch_stage_f64_batched(const Batch& b, int scheme, int shape, cudaStream_t st);
 inline void shape_tile(bool fp64, int shape, int* tj, int* tk)
 {
   *tk = shape == 1 ? 16 : 32;

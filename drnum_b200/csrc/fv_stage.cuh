@@ -359,12 +359,12 @@ struct StageLaunch {
 };
 
 // One patch per launch: grid (k tiles, j tiles, i chunks).
-template <class Policy, int TJ, int TK>
+template <class Policy, class Scheme, int TJ, int TK>
 __global__ void __launch_bounds__(TJ * TK, F64Occupancy<TJ * TK>::min_blocks)
 fv_stage_kernel(const __grid_constant__ StageLaunch<Policy> L)
 {
   const int i0 = blockIdx.z * L.a.g.i_chunk;
-  fv_stage_tile<Policy, AusmPlusFace, TJ, TK>(L.a, L.tma ? &L.tm : nullptr, blockIdx.y * TJ, blockIdx.x * TK, i0,
+  fv_stage_tile<Policy, Scheme, TJ, TK>(L.a, L.tma ? &L.tm : nullptr, blockIdx.y * TJ, blockIdx.x * TK, i0,
                                 min(L.a.g.ni, i0 + L.a.g.i_chunk));
 }
 
