@@ -191,11 +191,49 @@ struct dn_ctx {
   void* stage_user = nullptr;
 };
 
-#ifndef DN_FX_WAVE_CTAS
-#define DN_FX_WAVE_CTAS 2   // CTAs per SM counted in a wave when sizing FX32 plane ranges
-#endif
-
 namespace {
+
+// Planes per CTA of a single-patch launch: the range whose launch takes the
+// least time when a CTA's planes take 1 + share * r each (r CTAs resident on
+// its SM), prolog of them are spent on its prologue, and CTAs beyond a wave
+// wait for it.  Short ranges give a small patch the CTAs to fill the GPU (a
+// CTA's planes are a serial chain), long ones spend less on prologues, and
+// the last wave decides between them.  Fitted to both kernels on eleven
+// patches of 16^3 to 40 x 200 x 200 cells with ranges of 1 to 86 planes: the
+// choice is within 3 % of the best measured range but for two (FP32 40 x 200
+// x 200 22 %, FP64 97 x 61 x 83 8 %).  Against the fixed rule before (about four
+// waves of at least eight planes), us a stage: FP32 16^3 39.0 -> 10.4, 32^3
+// 34.9 -> 10.4, 64^3 32.9 -> 18.6; FP64 16^3 68 -> 14.7, 32^3 70.4 -> 17.5,
+// 64^3 82.3 -> 60.7.
+struct ChunkCost {
+  int ctas_per_sm;   // resident CTAs of the kernel
+  double prolog;     // prologue in planes
+  double share;      // slowdown of a plane per resident CTA
+};
+constexpr ChunkCost kChunkF64 = {4, 0.25, 0.2};
+constexpr ChunkCost kChunkFx32 = {2, 1.5, 0.5};
+int default_i_chunk(int ni, int nj, int nk, int tj, int tk, int num_sms, const ChunkCost& k)
+{
+  const long tiles = (long)((nj + tj - 1) / tj) * ((nk + tk - 1) / tk);
+  const long wave = (long)num_sms * k.ctas_per_sm;
+  double best = -1;
+  int best_ic = ni;
+  for (int ic = (ni + 65534) / 65535; ic <= ni;) {   // (the grid's third extent is 16 bits)
+    const int chunks = (ni + ic - 1) / ic;
+    const long n = tiles * chunks;
+    const long rest = n % wave;
+    double t = (double)(n / wave) * (1.0 + k.share * k.ctas_per_sm);
+    if (rest) t += 1.0 + k.share * (double)((rest + num_sms - 1) / num_sms);
+    t *= ic + k.prolog;
+    if (best < 0 || t < best) {
+      best = t;
+      best_ic = ic;
+    }
+    if (chunks == 1) break;
+    ic = (ni + chunks - 2) / (chunks - 1);   // the shortest range with a chunk less
+  }
+  return best_ic;
+}
 
 constexpr int kSumThreads = 256;
 constexpr int kSumBlocks = 1184;   // 8 per SM on 148 SMs; fixed => deterministic order
@@ -1531,7 +1569,7 @@ int stage_patch(dn_ctx* c, DnPatch& p, int in_b, int un_b, int out_b, double fac
     a.active = p.active;
     a.err = c->d_err;
     a.err_info = c->d_err_info;
-    g.i_chunk = dn::default_i_chunk(g.ni, g.nj, g.nk, 4, 32, c->num_sms, 3);
+    g.i_chunk = default_i_chunk(g.ni, g.nj, g.nk, 4, 32, c->num_sms, kChunkF64);
     a.g = g;
     a.p.Ax = dy * dz; a.p.Ay = dx * dz; a.p.Az = dx * dy; a.p.pf = pf;
     a.wall = p.wall;
@@ -1549,7 +1587,7 @@ int stage_patch(dn_ctx* c, DnPatch& p, int in_b, int un_b, int out_b, double fac
     a.g.ni = g.ni; a.g.nj = g.nj; a.g.nk = g.nk; a.g.kp = p.kp;
     a.g.per_x = g.per_x; a.g.per_y = g.per_y; a.g.per_z = g.per_z;
     a.g.i_chunk = p.i_chunk > 0 ? std::min(p.i_chunk, g.ni)
-                                : dn::default_i_chunk(g.ni, g.nj, g.nk, tj, tk, c->num_sms, DN_FX_WAVE_CTAS);
+                                : default_i_chunk(g.ni, g.nj, g.nk, tj, tk, c->num_sms, kChunkFx32);
     dn::fx_set_params(a.p, dx, dy, dz, factor, p.base, p.quantum);
     a.wall = p.wall;
     e = dn::launch_stage_fx32(a, c->stream);
@@ -3015,11 +3053,11 @@ int dn_autotune(dn_ctx* c, const char* cache_path, double cost_out[DN_NUM_TILE_S
       if (!P.owned) continue;
       int tj, tk;
       dn::fx32_tile(&tj, &tk);
-      const int def = dn::default_i_chunk(P.d.ni, P.d.nj, P.d.nk, tj, tk, c->num_sms, DN_FX_WAVE_CTAS);
-      const int cand[6] = {def, 16, 24, 32, 48, 64};
+      const int def = default_i_chunk(P.d.ni, P.d.nj, P.d.nk, tj, tk, c->num_sms, kChunkFx32);
+      const int cand[11] = {def, 8, 12, 16, 20, 24, 28, 32, 40, 48, 64};
       int best = def;
       double best_ms = 1e300;
-      for (int k = 0; k < 6; ++k) {
+      for (int k = 0; k < 11; ++k) {
         if (cand[k] > P.d.ni || (k > 0 && cand[k] == def)) continue;
         P.i_chunk = cand[k];
         int st = DN_OK;

@@ -113,17 +113,4 @@ cudaError_t launch_stage_fx32_batched(const Batch& b, int shape, int form, cudaS
   return launch_fx_batched_shape<kFxEdge>(b, shape, st);
 }
 
-int default_i_chunk(int ni, int nj, int nk, int tj, int tk, int num_sms, int ctas_per_sm)
-{
-  const long tiles = (long)((nj + tj - 1) / tj) * ((nk + tk - 1) / tk);
-  const long want = (long)num_sms * ctas_per_sm * 4;   // about four waves
-  long chunks = (want + tiles - 1) / tiles;
-  if (chunks < 1) chunks = 1;
-  long ic = (ni + chunks - 1) / chunks;
-  if (ic < 8) ic = 8;                                   // amortise the 4-plane prologue
-  if (ic > ni) ic = ni;
-  return (int)ic;
-}
-
-
 } // namespace dn

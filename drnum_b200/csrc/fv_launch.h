@@ -46,7 +46,4 @@ inline void shape_tile(bool fp64, int shape, int* tj, int* tk)
   else *tj = shape == 0 ? 8 : 16;
 }
 
-// Chooses the i-chunk so that the grid holds enough CTAs to fill the GPU.
-int default_i_chunk(int ni, int nj, int nk, int tj, int tk, int num_sms, int ctas_per_sm);
-
 } // namespace dn
