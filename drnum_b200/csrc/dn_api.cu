@@ -157,6 +157,7 @@ struct dn_ctx {
   // deals the work to that many waves of persistent CTAs; 0 launches one
   // CTA per work item, items of at least batch_min_planes planes
   int batch_min_planes = 8;
+  bool batch_auto = true;   // FP64: plane ranges by the cost model until a shortest range is set
   int batch_waves = 2;
   cudaStream_t s_aux = nullptr;               // second branch of a batched stage (inside and edge tiles)
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -210,29 +211,44 @@ struct ChunkCost {
   double prolog;     // prologue in planes
   double share;      // slowdown of a plane per resident CTA
 };
-constexpr ChunkCost kChunkF64 = {4, 0.25, 0.2};
+constexpr ChunkCost kChunkF64 = {4, 0.25, 0.2};          // 4 x 32 and 8 x 16 tiles
+constexpr ChunkCost kChunkF64Wide = {2, 0.25, 0.4};      // 8 x 32 tiles
 constexpr ChunkCost kChunkFx32 = {2, 1.5, 0.5};
-int default_i_chunk(int ni, int nj, int nk, int tj, int tk, int num_sms, const ChunkCost& k)
+// time of n CTAs in whole waves, in planes of a CTA alone
+double wave_time(long n, int num_sms, const ChunkCost& k)
 {
-  const long tiles = (long)((nj + tj - 1) / tj) * ((nk + tk - 1) / tk);
-  const long wave = (long)num_sms * k.ctas_per_sm;
+  const long wave = (long)num_sms * k.ctas_per_sm, rest = n % wave;
+  double t = (double)(n / wave) * (1.0 + k.share * k.ctas_per_sm);
+  if (rest) t += 1.0 + k.share * (double)((rest + num_sms - 1) / num_sms);
+  return t;
+}
+
+// the range for `tiles` column tiles each of several extents (ni, tiles)
+int best_range(const std::vector<std::pair<int, long>>& runs, int num_sms, const ChunkCost& k)
+{
+  int ni = 1;
+  for (const auto& r : runs) ni = std::max(ni, r.first);
   double best = -1;
   int best_ic = ni;
-  for (int ic = (ni + 65534) / 65535; ic <= ni;) {   // (the grid's third extent is 16 bits)
-    const int chunks = (ni + ic - 1) / ic;
-    const long n = tiles * chunks;
-    const long rest = n % wave;
-    double t = (double)(n / wave) * (1.0 + k.share * k.ctas_per_sm);
-    if (rest) t += 1.0 + k.share * (double)((rest + num_sms - 1) / num_sms);
-    t *= ic + k.prolog;
+  for (int ic = (ni + 65534) / 65535; ic <= ni;) {   // (a grid's third extent is 16 bits)
+    long n = 0;
+    for (const auto& r : runs) n += r.second * ((r.first + ic - 1) / ic);
+    const double t = wave_time(n, num_sms, k) * (ic + k.prolog);
     if (best < 0 || t < best) {
       best = t;
       best_ic = ic;
     }
+    const int chunks = (ni + ic - 1) / ic;
     if (chunks == 1) break;
     ic = (ni + chunks - 2) / (chunks - 1);   // the shortest range with a chunk less
   }
   return best_ic;
+}
+
+int default_i_chunk(int ni, int nj, int nk, int tj, int tk, int num_sms, const ChunkCost& k)
+{
+  const long tiles = (long)((nj + tj - 1) / tj) * ((nk + tk - 1) / tk);
+  return best_range({{ni, tiles}}, num_sms, k);
 }
 
 constexpr int kSumThreads = 256;
@@ -1223,7 +1239,7 @@ int default_shape(const DnPatch& p)
 constexpr double kProlog = 3.0;
 constexpr int kMinPiece = 4;
 
-void deal_greedy(const std::vector<dn::WorkItem>& runs, double target, std::vector<dn::WorkItem>& items,
+void deal_greedy(const std::vector<dn::WorkItem>& runs, double target, int kMinPiece, std::vector<dn::WorkItem>& items,
                  std::vector<int>& groups)
 {
   items.clear();
@@ -1248,15 +1264,32 @@ void deal_greedy(const std::vector<dn::WorkItem>& runs, double target, std::vect
   groups.push_back((int)items.size());
 }
 
-void deal_runs(const std::vector<dn::WorkItem>& runs, int slots, std::vector<dn::WorkItem>& items,
+// Too few planes for that (under 2 kMinPiece a CTA): the number of CTAs, in
+// whole CTAs per SM, that the cost model of single-patch launches predicts
+// fastest, down to pieces of a plane.  (A 66 x 64 x 64 sphere pair ran 82 and
+// 50 CTAs of eight planes on 148 SMs.)
+void deal_runs(const std::vector<dn::WorkItem>& runs, int slots, int num_sms, std::vector<dn::WorkItem>& items,
                std::vector<int>& groups)
 {
   long planes = 0;
   for (const auto& r : runs) planes += r.i1 - r.i0;
-  const long want = std::max(1L, std::min<long>(slots, planes / (2 * kMinPiece)));
+  long want = slots;
+  int piece = kMinPiece;
+  if (planes < (long)slots * 2 * kMinPiece) {
+    double best = -1;
+    for (long n = num_sms; n <= slots; n += num_sms) {
+      const long m = std::min(n, planes);
+      const double t = wave_time(m, num_sms, kChunkFx32) * ((double)planes / (double)m + kChunkFx32.prolog);
+      if (best < 0 || t < best) {
+        best = t;
+        want = m;
+      }
+    }
+    piece = (int)std::max(1L, std::min<long>(kMinPiece, planes / want));
+  }
   double target = ((double)planes + kProlog * (double)want) / (double)want;
   for (int k = 0; k < 400; ++k) {
-    deal_greedy(runs, target, items, groups);
+    deal_greedy(runs, target, piece, items, groups);
     if ((long)groups.size() - 1 <= want) return;
     target *= 1.01;
   }
@@ -1365,6 +1398,18 @@ int build_batch(dn_ctx* c)
   // launch per form keeps one code path per kernel
   std::vector<dn::WorkItem> items[3][dn::kNumShapes];
   std::vector<int> groups[3][dn::kNumShapes];
+  // FP64 without a set shortest range: a tile shape's launch takes the range
+  // of the cost model
+  int range64[dn::kNumShapes] = {};
+  if (fp64 && c->batch_auto) {
+    std::vector<std::pair<int, long>> runs[dn::kNumShapes];
+    for (size_t q = 0; q < np; ++q) {
+      const DnPatch& P = c->patches[q];
+      if (P.owned && P.patch_active) runs[c->shape[q]].emplace_back(P.d.ni, (long)ptiles[q].size());
+    }
+    for (int sh = 0; sh < dn::kNumShapes; ++sh)
+      if (!runs[sh].empty()) range64[sh] = best_range(runs[sh], c->num_sms, sh == 2 ? kChunkF64Wide : kChunkF64);
+  }
   for (size_t q = 0; q < np; ++q) {
     const DnPatch& P = c->patches[q];
     if (!P.owned || !P.patch_active) continue;
@@ -1374,6 +1419,7 @@ int build_batch(dn_ctx* c)
     const bool persistent = !fp64 && c->batch_waves > 0;
     long ic = (P.d.ni + chunks - 1) / chunks;
     if (ic < c->batch_min_planes) ic = c->batch_min_planes;   // amortise each item's 3-plane prologue
+    if (range64[c->shape[q]]) ic = range64[c->shape[q]];
     if (ic > P.d.ni || persistent) ic = P.d.ni;
     for (int i0 = 0; i0 < P.d.ni; i0 += (int)ic)
       for (const TileRef& t : ptiles[q]) {
@@ -1395,7 +1441,7 @@ int build_batch(dn_ctx* c)
         cudaError_t e = dn::fx32_batched_occupancy(q, f, &occ);
         if (e != cudaSuccess) return cuda_fail(c, e, "batched stage occupancy");
         const std::vector<dn::WorkItem> runs = items[f][q];
-        deal_runs(runs, c->num_sms * std::max(1, occ) * c->batch_waves, items[f][q], groups[f][q]);
+        deal_runs(runs, c->num_sms * std::max(1, occ) * c->batch_waves, c->num_sms, items[f][q], groups[f][q]);
       }
     }
   }
@@ -2634,6 +2680,7 @@ int dn_set_option(dn_ctx* c, int option, int value)
     if (value < (option == DN_OPT_BATCH_WAVES ? 0 : 1) || value > 64)
       return fail(c, DN_ERR_ARG, "schedule option %d out of range: %d", option, value);
     (option == DN_OPT_BATCH_WAVES ? c->batch_waves : c->batch_min_planes) = value;
+    if (option == DN_OPT_BATCH_MIN_PLANES) c->batch_auto = false;
     c->batch_dirty = true;
     c->generation++;
     return DN_OK;
@@ -3102,31 +3149,69 @@ int dn_autotune(dn_ctx* c, const char* cache_path, double cost_out[DN_NUM_TILE_S
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     const bool fp64 = c->precision == DN_FP64;
-    // (waves, shortest item): persistent waves for FP32 bulk, or one CTA per item
-    const int cand64[5][2] = {{0, 8}, {0, 16}, {0, 24}, {0, 32}, {0, 48}};
-    const int cand32[8][2] = {{0, 8}, {0, 16}, {0, 24}, {0, 32}, {0, 48}, {1, 8}, {2, 8}, {4, 8}};
-    const int n_cand = fp64 ? 5 : 8;
+    // (waves, shortest item): persistent waves for FP32 bulk, or one CTA per
+    // item; 0, 0: FP64 ranges by the cost model
+    const int cand64[4][2] = {{0, 0}, {0, 8}, {0, 16}, {0, 32}};
+    const int cand32[5][2] = {{1, 8}, {2, 8}, {4, 8}, {0, 8}, {0, 16}};
+    const int n_cand = fp64 ? 4 : 5;
+    // with the shapes chosen per patch, and with the one shape that is
+    // fastest for all of them: the costs were measured with one schedule, and
+    // shapes and schedule together decide (level-set sphere 732 us a step
+    // when the schedule was tuned for the per-patch shapes only, 699 with
+    // 16 x 32 tiles in one wave)
+    std::vector<std::vector<int>> shapes(1, c->shape);
+    {
+      int u = 0;
+      double best_u = 1e300;
+      for (int sh = 0; sh < dn::kNumShapes; ++sh) {
+        double t = 0;
+        for (size_t q = 0; q < c->patches.size(); ++q)
+          if (c->patches[q].owned) t += cost[sh] * padded_cells(c, c->patches[q], sh);
+        if (t < best_u) { best_u = t; u = sh; }
+      }
+      for (int sh = 0; sh < dn::kNumShapes; ++sh) {
+        // 16 x 32 tiles too (FP32): fewest halo cells
+        if (sh != u && (fp64 || sh != 2)) continue;
+        std::vector<int> all(c->shape.size(), sh);
+        if (std::find(shapes.begin(), shapes.end(), all) == shapes.end()) shapes.push_back(all);
+      }
+    }
+    std::vector<int> best_s = c->shape;
     int best_w = c->batch_waves, best_p = c->batch_min_planes;
+    bool best_a = c->batch_auto;
     double best_ms = 1e300;
     int st = DN_OK;
-    for (int k = 0; k < n_cand && st == DN_OK; ++k) {
-      c->batch_waves = fp64 ? cand64[k][0] : cand32[k][0];
-      c->batch_min_planes = fp64 ? cand64[k][1] : cand32[k][1];
-      c->batch_dirty = true;
-      for (int r = 0; r < 5 && st == DN_OK; ++r) {
-        if (r == 2) cudaEventRecord(e0, c->stream);
-        st = stage_all(c, c->fmap[0], c->fmap[1], c->fmap[2], 0.0);
+    for (size_t m = 0; m < shapes.size() && st == DN_OK; ++m) {
+      for (int k = 0; k < n_cand && st == DN_OK; ++k) {
+        c->shape = shapes[m];
+        c->batch_waves = fp64 ? cand64[k][0] : cand32[k][0];
+        const int mp = fp64 ? cand64[k][1] : cand32[k][1];
+        c->batch_auto = mp == 0;
+        c->batch_min_planes = mp ? mp : 8;
+        c->batch_dirty = true;
+        for (int r = 0; r < 5 && st == DN_OK; ++r) {
+          if (r == 2) cudaEventRecord(e0, c->stream);
+          st = stage_all(c, c->fmap[0], c->fmap[1], c->fmap[2], 0.0);
+        }
+        cudaEventRecord(e1, c->stream);
+        cudaEventSynchronize(e1);
+        float ms = 0;
+        cudaEventElapsedTime(&ms, e0, e1);
+        if (st == DN_OK && ms < best_ms) {
+          best_ms = ms;
+          best_s = c->shape;
+          best_w = c->batch_waves;
+          best_p = c->batch_min_planes;
+          best_a = c->batch_auto;
+        }
       }
-      cudaEventRecord(e1, c->stream);
-      cudaEventSynchronize(e1);
-      float ms = 0;
-      cudaEventElapsedTime(&ms, e0, e1);
-      if (st == DN_OK && ms < best_ms) { best_ms = ms; best_w = c->batch_waves; best_p = c->batch_min_planes; }
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    c->shape = best_s;
     c->batch_waves = best_w;
     c->batch_min_planes = best_p;
+    c->batch_auto = best_a;
     c->batch_dirty = true;
     c->generation++;
     if (st != DN_OK) return st;
