@@ -48,12 +48,17 @@ namespace dn {
 struct Guard {
   static constexpr int exp_hi(int e) { return (1023 + e) << 20; }   // high word of 2^e
   unsigned mant = 0;           // largest upper-significand field of a denominator
-  unsigned dmax = 0;           // largest |difference|
+  float dmax = 0.0f;           // largest |difference|: its high word read as a float (same order; NaN stays)
   unsigned zmin = 0xffffffffu; // smallest nonzero numerator (high word - 1: zero wraps to the top)
   int lo = 0x7fffffff, hi = 0; // extrema of what must be positive
   bool minus_zero = false;     // a difference of -0 (or a denormal next to it)
   __device__ __forceinline__ void den(double b) { mant = max(mant, (unsigned)__double2hiint(b) & 0xfffffu); }
-  __device__ __forceinline__ void diff(double x) { dmax = max(dmax, (unsigned)__double2hiint(x) & 0x7fffffffu); }
+  __device__ __forceinline__ void diff(double x, double y)
+  {
+    asm("max.NaN.f32 %0, %1, %2, %3;"
+        : "=f"(dmax) : "f"(dmax), "f"(fabsf(__int_as_float(__double2hiint(x)))),
+          "f"(fabsf(__int_as_float(__double2hiint(y)))));
+  }
   __device__ __forceinline__ void num(double x) { zmin = min(zmin, ((unsigned)__double2hiint(x) & 0x7fffffffu) - 1u); }
   __device__ __forceinline__ void positive(double x)
   {
@@ -64,7 +69,7 @@ struct Guard {
   // least 1e-10, positive quantities in [2^-300, 2^300] (NaN is outside)
   __device__ __forceinline__ bool any() const
   {
-    return mant == 0xfffffu || dmax >= (unsigned)exp_hi(400) || zmin < (unsigned)exp_hi(-500) || lo < exp_hi(-300) ||
+    return mant == 0xfffffu || !(dmax < __int_as_float(exp_hi(400))) || zmin < (unsigned)exp_hi(-500) || lo < exp_hi(-300) ||
            hi >= exp_hi(300) || minus_zero;
   }
 };
@@ -112,16 +117,16 @@ struct Recip {
 template <int N>
 __device__ __forceinline__ void half_van_albada(const double (&d1)[N], const double (&d2)[N], double (&out)[N], Guard& g)
 {
-  // non_zero by bit patterns: |d1| < eps (as integers) becomes eps with the
-  // sign of d1 (-0, which counts as positive, is left to the guard)
+  // non_zero: |d1| < eps becomes eps with the sign of d1 (-0, which counts as
+  // positive, is left to the guard)
   constexpr unsigned long long eps = 0x3ddb7cdfd9d7bdbbull;     // 1e-10
   double b[N], y[N], e[N], q[N], num[N];
   #pragma unroll
   for (int c = 0; c < N; ++c) {
     const int h = __double2hiint(d1[c]);
     g.minus_zero |= h == (int)0x80000000;
-    g.diff(d1[c]);
-    const bool small = ((unsigned long long)__double_as_longlong(d1[c]) & 0x7fffffffffffffffull) < eps;
+    if (c & 1) g.diff(d1[c], d1[c - 1]);
+    const bool small = fabs(d1[c]) < 1e-10;
     b[c] = __hiloint2double(small ? ((int)(eps >> 32) | (h & (int)0x80000000)) : h,
                             small ? (int)(unsigned)eps : __double2loint(d1[c]));
     g.den(b[c]);
@@ -207,9 +212,11 @@ __device__ __forceinline__ void limited_states(const FaceCells& f, double vl[5],
     d1[2 * v + 1] = __dsub_rn(vr[v], f.p1[v * S]);
     d2[2 * v] = d;
     d2[2 * v + 1] = -d;
-    g.diff(d);
     g.num(d);
   }
+  g.diff(d2[0], d2[2]);
+  g.diff(d2[4], d2[6]);
+  g.diff(d2[8], d2[8]);
   half_van_albada(d1, d2, h, g);
   #pragma unroll
   for (int v = 0; v < 5; ++v) {
