@@ -260,19 +260,71 @@ __device__ __forceinline__ int fx_quant1(float x, FaceRange& r)
   return __float2int_rn(x);
 }
 
-// Patch-face flux of side `side` (axis AXIS) of a boundary cell with FP32
-// state U, in whole quanta (0 for a zero-flux side), recorded in r.  Placed
-// in the face arrays where the missing interior face would be, a min side's
-// flux counts as the face below the cell and a max side's as the face above
-// it, so the residual adds it with the reference's signs (+ min, - max).
-template <int AXIS>
+// Patch-face flux of side `side` (axis side/2) of a boundary cell with FP32
+// state U, in whole quanta (0 for a zero-flux side), recorded in r: the
+// operations of wall_flux<axis> with the axis chosen at run time.  One copy
+// of this code per call site, in loops that are not unrolled: a copy per
+// axis, side and cell of a pair (twelve in the residual of an edge tile)
+// filled the instruction cache (the single-patch kernel waited for
+// instructions: no_instruction 4.4 of 11.6 warps per issue on a closed 125 x
+// 67 x 93 patch) and spilled (inside form of 16 x 32 tiles 268 bytes a
+// thread, now 72).  Measured together with every side in the slot of the
+// missing face: closed 125 x 67 x 93 patch 79 -> 69 us a stage, 160^3 233 ->
+// 197; RK steps of the jet 1588 -> 1548 us, sphere 704 -> 691, 64 uneven
+// patches 1988 -> 1890.
 __device__ __forceinline__ void fx_wall_quanta(const WallBC& bc, int side, int face, const float U[5], float A,
                                                const float2* face_scale, FaceRange& r, int q[5])
 {
-  float F[5];
-  const bool on = wall_flux<AXIS>(bc, side, face, U, A, F);
+  const int axis = side >> 1, kind = bc.kind[side];
+  if (kind == kWallZero) {
+    #pragma unroll
+    for (int v = 0; v < 5; ++v) q[v] = 0;
+    return;
+  }
+  float p1, T1, u1, v1, w1;
+  wall_prim(U, p1, T1, u1, v1, w1);
+  float F[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+  float p = p1;
+  if (kind != kWallSlip) {
+    float Tt = T1, u = u1, v = v1, w = w1;
+    if (kind == kWallInflow) {
+      const double* e = bc.table[side] + (size_t)face * 5;
+      if (e[0] == e[0]) p = (float)e[0];         // NaN: pressure of the boundary cell
+      Tt = (float)e[1];
+      u = (float)e[2];
+      v = (float)e[3];
+      w = (float)e[4];
+    } else {
+      const double* f = bc.ff[side];
+      const float u0 = (float)f[2], v0 = (float)f[3], w0 = (float)f[4], a0 = (float)f[5];
+      const float a1 = sqrtf(float(Gas::gamma) * float(Gas::R) * T1);
+      float M0 = (axis == 0 ? u0 : (axis == 1 ? v0 : w0)) / a0;
+      float M1 = (axis == 0 ? u1 : (axis == 1 ? v1 : w1)) / a1;
+      if (side & 1) {
+        M0 = -M0;
+        M1 = -M1;
+      }
+      const float M = 0.5f * (M0 + M1);
+      if (M >= 0.0f) {
+        if (M >= 1.0f) p = (float)f[0];
+        Tt = (float)f[1];
+        u = u0;
+        v = v0;
+        w = w0;
+      }
+    }
+    F[0] = A * p / (float(Gas::R) * Tt) * (axis == 0 ? u : (axis == 1 ? v : w));
+    F[1] = F[0] * u;
+    F[2] = F[0] * v;
+    F[3] = F[0] * w;
+    F[4] = F[0] * (float(kGasCp) * Tt + 0.5f * (u * u + v * v + w * w));
+  }
+  const float Ap = A * p;
+  F[1] = axis == 0 ? F[1] + Ap : F[1];
+  F[2] = axis == 1 ? F[2] + Ap : F[2];
+  F[3] = axis == 2 ? F[3] + Ap : F[3];
   #pragma unroll
-  for (int v = 0; v < 5; ++v) q[v] = on ? fx_quant1(F[v] * face_scale[v].x, r) : 0;
+  for (int v = 0; v < 5; ++v) q[v] = fx_quant1(F[v] * face_scale[v].x, r);
 }
 
 // Cell whose state stands at index x of an axis: the wrapped cell on a
@@ -467,18 +519,27 @@ __device__ __forceinline__ bool fx_stage_tile_impl(const FxArgs& a, const CUtens
   const int tid = ty * TP + tp;
   const int kk = 2 * tp;                          // tile column of the pair's first cell
   const int j = j0 + ty, ka = k0 + kk, kb = ka + 1;
-  // inside tiles place the y and z patch-face fluxes of their boundary cells
-  // in the face arrays, in the slot of the missing face, during the slope
-  // phase (their state is in the ring then); the face phase leaves those
-  // slots alone and the residual sums them like interior faces.  The slots
-  // are written and read by the same thread.
-  const bool yz_walls = WALLS && MODE == kFxInside && a.wall.any;
-  const bool w_ymin = yz_walls && j == 0 && !g.per_y && g.nj > 2;
-  const bool w_ymax = yz_walls && j == g.nj - 1 && !g.per_y && g.nj > 2;
-  const bool w_zmin = yz_walls && ka == 0 && !g.per_z && g.nk > 2;
-  const bool w_zmax = yz_walls && kb == g.nk - 1 && !g.per_z && g.nk > 2;
   const bool own_a = PAIRS || ((j < g.nj) && (ka < g.nk));
   const bool own_b = PAIRS || ((j < g.nj) && (kb < g.nk));
+  // Patch-face fluxes stand where the missing face of a boundary cell would,
+  // and the residual sums them like interior faces (whole quanta; a cell
+  // still sums six).  The y and z sides go into the face arrays during the
+  // slope phase, when the cell's state is in the ring, and the face phase
+  // leaves those slots alone; the x sides replace the column's first lower
+  // and last upper face in the residual.  Full tiles have x sides only.
+  const bool yz_walls = WALLS && !FULL && a.wall.any;
+  const bool y_walls = yz_walls && !g.per_y && g.nj > 2, z_walls = yz_walls && !g.per_z && g.nk > 2;
+  const bool w_ymin = y_walls && j == 0 && own_a;
+  const bool w_ymax = y_walls && j == g.nj - 1 && own_a;
+  const bool w_zmin = z_walls && ka == 0 && own_a;
+  const bool w_zmax = z_walls && kb == g.nk - 1 && own_b;
+  const bool w_zmaxa = !PAIRS && z_walls && ka == g.nk - 1 && own_a;   // the pair's first cell is the last column
+  // slots of this thread's own faces that hold a patch face: the y face
+  // below row 0, or below the row after the last; the z face below the
+  // pair's first cell likewise, or below its second
+  const bool keep_y = w_ymin || (!PAIRS && y_walls && j == g.nj);
+  const bool keep_za = w_zmin || (!PAIRS && z_walls && ka == g.nk);
+  const bool keep_zb = w_zmaxa;
   const int njk = g.nj * g.kp;                    // plane stride (rows of kp elements)
   const int nc = g.ni * njk;                      // variable stride (5 * nc < 2^31, host check)
   // TMA boxes start at x = k0-4 (main; a multiple of 4 int32 since TK is),
@@ -780,32 +841,25 @@ __device__ __forceinline__ bool fx_stage_tile_impl(const FxArgs& a, const CUtens
       }
     }
     FaceRange wmag_yz;   // y and z patch-face fluxes of the own cells
-    if (w_ymin || w_ymax || w_zmin || w_zmax) {
-      float Ua[5], Ub[5];
-      #pragma unroll
-      for (int v = 0; v < 5; ++v) {
-        const float2 u = RP(r0, v, 0, 0);
-        Ua[v] = u.x;
-        Ub[v] = u.y;
-      }
-      int qa[5], qb[5];
-      if (w_ymin || w_ymax) {
-        const int side = w_ymin ? 2 : 3;
-        fx_wall_quanta<1>(a.wall, side, i * g.nk + ka, Ua, P.A[1].x, P.face_scale, wmag_yz, qa);
-        fx_wall_quanta<1>(a.wall, side, i * g.nk + kb, Ub, P.A[1].x, P.face_scale, wmag_yz, qb);
+    if (w_ymin || w_ymax || w_zmin || w_zmax || w_zmaxa) {
+      // the y side of the pair's cells (t = 0, 1), the z side of one of them (2)
+      #pragma unroll 1
+      for (int t = w_ymin || w_ymax ? 0 : 2; t < (w_zmin || w_zmax || w_zmaxa ? 3 : 2); ++t) {
+        const bool ydir = t < 2;
+        const int second = ydir ? t : (w_zmax ? 1 : 0);
+        if (!PAIRS && ydir && second && !own_b) continue;
+        float U[5];
+        int q[5];
         #pragma unroll
-        for (int v = 0; v < 5; ++v)
-          *reinterpret_cast<int2*>(&sm.qy[v][w_ymin ? ty : ty + 1][kk]) = make_int2(qa[v], qb[v]);
-      }
-      if (w_zmin) {
-        fx_wall_quanta<2>(a.wall, 4, i * g.nj + j, Ua, P.A[2].x, P.face_scale, wmag_yz, qa);
+        for (int v = 0; v < 5; ++v) U[v] = r0[v * VS + second];
+        fx_wall_quanta(a.wall, ydir ? (w_ymin ? 2 : 3) : (w_zmin ? 4 : 5), ydir ? i * g.nk + ka + second : i * g.nj + j,
+                       U, ydir ? P.A[1].x : P.A[2].x, P.face_scale, wmag_yz, q);
+        // (z max above the pair's first cell: the slot of the face between the cells)
+        int* const dst = ydir ? &sm.qy[0][w_ymin ? ty : ty + 1][kk + second]
+                              : (w_zmaxa ? &sm.qz[0][ty][tp].y : &sm.qz[0][ty][w_zmin ? tp : tp + 1].x);
+        const int stride = ydir ? (TJ + 1) * TK : TJ * (TP + 1) * 2;
         #pragma unroll
-        for (int v = 0; v < 5; ++v) sm.qz[v][ty][tp].x = qa[v];
-      }
-      if (w_zmax) {
-        fx_wall_quanta<2>(a.wall, 5, i * g.nj + j, Ub, P.A[2].x, P.face_scale, wmag_yz, qb);
-        #pragma unroll
-        for (int v = 0; v < 5; ++v) sm.qz[v][ty][tp + 1].x = qb[v];
+        for (int v = 0; v < 5; ++v) dst[v * stride] = q[v];
       }
     }
     __syncthreads();
@@ -846,7 +900,7 @@ __device__ __forceinline__ bool fx_stage_tile_impl(const FxArgs& a, const CUtens
         int2 q = fx_quant2(mul2(F[v], P.face_scale[v]), fmag);
         if (!exa) q.x = 0;
         if (!exb) q.y = 0;
-        if (!w_ymin) *reinterpret_cast<int2*>(&sm.qy[v][ty][kk]) = q;   // else: the patch face, placed before
+        if (!keep_y) *reinterpret_cast<int2*>(&sm.qy[v][ty][kk]) = q;   // else: the patch face, placed before
       }
     }
     // z faces below the pair's two cells
@@ -867,7 +921,8 @@ __device__ __forceinline__ bool fx_stage_tile_impl(const FxArgs& a, const CUtens
         int2 q = fx_quant2(mul2(F[v], P.face_scale[v]), fmag);
         if (!exa) q.x = 0;
         if (!exb) q.y = 0;
-        if (w_zmin) sm.qz[v][ty][tp].y = q.y;   // .x: the patch face, placed before
+        if (keep_za) sm.qz[v][ty][tp].y = q.y;   // .x: the patch face, placed before
+        else if (keep_zb) sm.qz[v][ty][tp].x = q.x;
         else sm.qz[v][ty][tp] = q;
       }
     }
@@ -893,7 +948,7 @@ __device__ __forceinline__ bool fx_stage_tile_impl(const FxArgs& a, const CUtens
           exb = ey && (PAIRS || k0 + c + 1 < g.nk);
         }
         // (the last row's patch face, if any, is placed by its own cells)
-        const bool keep = yz_walls && j0 + TJ == g.nj && !g.per_y && g.nj > 2;
+        const bool keep = y_walls && j0 + TJ == g.nj;
         #pragma unroll
         for (int v = 0; v < 5; ++v) {
           int2 q = fx_quant2(mul2(F[v], P.face_scale[v]), fmag);
@@ -919,7 +974,7 @@ __device__ __forceinline__ bool fx_stage_tile_impl(const FxArgs& a, const CUtens
           exb = ez && (PAIRS || j0 + jb < g.nj);
         }
         // (the last column's patch face, if any, is placed by its own cells)
-        const bool keep = yz_walls && k0 + TK == g.nk && !g.per_z && g.nk > 2;
+        const bool keep = z_walls && k0 + TK == g.nk;
         #pragma unroll
         for (int v = 0; v < 5; ++v) {
           const int2 q = fx_quant2(mul2(F[v], P.face_scale[v]), fmag);
@@ -983,30 +1038,28 @@ __device__ __forceinline__ bool fx_stage_tile_impl(const FxArgs& a, const CUtens
         act_a = a.active[c] != 0;
         act_b = act_b && a.active[c + 1] != 0;
       }
-      // patch-face fluxes of boundary cells: whole quanta like the interior
-      // faces (a wall face replaces the cell's missing interior face, so a
-      // cell still sums six faces)
-      // (inside tiles: the y and z sides are in the face arrays already)
-      const bool any_wall = WALLS && a.wall.any;
-      const bool x_only = MODE == kFxInside;
-      const bool edge_i = any_wall && (i == 0 || i == g.ni - 1);
-      const bool edge_ijk = edge_i || (any_wall && !x_only && (j == 0 || j == g.nj - 1));
-      const bool wall_a = x_only ? edge_i : any_wall && (edge_ijk || ka == 0 || ka == g.nk - 1);
-      const bool wall_b = own_b && (x_only ? edge_i : any_wall && (edge_ijk || kb == g.nk - 1));
-      long long wa[5] = {0, 0, 0, 0, 0}, wb[5] = {0, 0, 0, 0, 0};
+      // x patch faces in place of the missing x face (the state re-read from
+      // the stage input: the ring slot of plane i receives plane i+3 below,
+      // with no barrier in between)
       FaceRange wmag;
-      if (wall_a || wall_b) {
-        #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          if (q == 0 ? !wall_a : !wall_b) continue;
-          // the cell's state, re-read from the stage input: the ring slot of
-          // plane i receives plane i+3 below, with no barrier in between
+      if (WALLS && a.wall.any && !g.per_x && g.ni > 2 && (i == 0 || i == g.ni - 1)) {
+        #pragma unroll 1
+        for (int q = 0; q < (own_b ? 2 : 1); ++q) {
           float uc[5];
+          int w[5];
           #pragma unroll
           for (int v = 0; v < 5; ++v) uc[v] = fmaf(P.quantum[v].x, (float)a.in[v * nc + c + q], P.base[v].x);
-          add_wall_fluxes(a.wall, g.ni, g.nj, g.nk, g.per_x, g.per_y, g.per_z, i, j, ka + q, uc, P.A[0].x, P.A[1].x,
-                          P.A[2].x, q == 0 ? wa : wb,
-                          [&](int v, float F) { return fx_quant1(F * P.face_scale[v].x, wmag); }, !x_only);
+          fx_wall_quanta(a.wall, i == 0 ? 0 : 1, j * g.nk + ka + q, uc, P.A[0].x, P.face_scale, wmag, w);
+          #pragma unroll
+          for (int v = 0; v < 5; ++v) {
+            if (i == 0) {
+              if (q == 0) qx_lo[v].x = w[v];
+              else qx_lo[v].y = w[v];
+            } else {
+              if (q == 0) qx_hi[v].x = w[v];
+              else qx_hi[v].y = w[v];
+            }
+          }
         }
         fbad |= !(wmag.mag() < kFxFaceLimit);
       }
@@ -1024,9 +1077,9 @@ __device__ __forceinline__ bool fx_stage_tile_impl(const FxArgs& a, const CUtens
           const int zhi = sm.qz[v][ty][tp + 1].x;
           const int2 un = *reinterpret_cast<const int2*>(&sm.un[v][ty][kk]);
           const unsigned ra = (unsigned)qx_lo[v].x - (unsigned)qx_hi[v].x + (unsigned)ylo.x - (unsigned)yhi.x +
-                              (unsigned)zlo.x - (unsigned)zlo.y + (unsigned)wa[v];
+                              (unsigned)zlo.x - (unsigned)zlo.y;
           const unsigned rb = (unsigned)qx_lo[v].y - (unsigned)qx_hi[v].y + (unsigned)ylo.y - (unsigned)yhi.y +
-                              (unsigned)zlo.y - (unsigned)zhi + (unsigned)wb[v];
+                              (unsigned)zlo.y - (unsigned)zhi;
           o[v].x = (int)((unsigned)un.x + ra);
           o[v].y = (int)((unsigned)un.y + rb);
         }
@@ -1040,8 +1093,8 @@ __device__ __forceinline__ bool fx_stage_tile_impl(const FxArgs& a, const CUtens
           const int2 zlo = sm.qz[v][ty][tp];
           const int zhi = sm.qz[v][ty][tp + 1].x;
           const int2 un = *reinterpret_cast<const int2*>(&sm.un[v][ty][kk]);
-          const long long ra = (long long)qx_lo[v].x - qx_hi[v].x + ylo.x - yhi.x + zlo.x - zlo.y + wa[v];
-          const long long rb = (long long)qx_lo[v].y - qx_hi[v].y + ylo.y - yhi.y + zlo.y - zhi + wb[v];
+          const long long ra = (long long)qx_lo[v].x - qx_hi[v].x + ylo.x - yhi.x + zlo.x - zlo.y;
+          const long long rb = (long long)qx_lo[v].y - qx_hi[v].y + ylo.y - yhi.y + zlo.y - zhi;
           const long long oa = (long long)un.x + ra, ob = (long long)un.y + rb;
           // results outside the range are clamped to its edge and flagged below
           o[v].x = (int)(oa >= kFxLimit ? kFxLimit : (oa <= -kFxLimit ? -kFxLimit : oa));
