@@ -17,30 +17,53 @@
 //     the constant 1/cv is a literal;
 //   - operands for which the sequence is not proven exact are noted in a
 //     Guard, and a face with any of them is evaluated again by the plain
-//     expressions (out of line; a lane in some 1e4 for the reciprocal's
-//     excluded denominators, none for flows in any usual range).
+//     expressions (out of line; a face in some 2e4 for the reciprocal's
+//     excluded denominators, no other for flows in any usual range).
 //
-// Exactness.  Let y be an approximation of 1/b.  By Markstein's theorems
-// (P. Markstein, IBM J. Res. Dev. 34, 1990; J.-M. Muller et al., Handbook of
-// Floating-Point Arithmetic, ch. 4) a quotient q within one ulp of a/b with
-// its exact residual r = a - b q gives fl(q + r y) = the correctly rounded
-// a/b when |b y - 1| is at most 2^-53 (1 + d) and the significand of y is
-// above 1 + d (the rounding error of r y then stays below the distance of
-// a/b from any midpoint of two doubles).  Recip's y is y0 (1 + e + e^2 +
-// e^3), e = 1 - b y0, from PTX's rcp.approx.ftz.f64 (relative error about
-// 2^-20, documented as working on the upper 32 bits): the truncation e^4 is
-// below 2^-72, so d is below 2^-18 and only denominators whose upper 20
-// significand bits are all ones are excluded.  The first quotient a y is
-// within 1.5 ulp, one residual step makes it faithful, the second correctly
-// rounds it.  Checked on the CPU against `/` on 3e8 operand pairs, half of
-// them next to a midpoint, with the seed off by up to two units of 2^-20.
+// Exactness (after Markstein's theorems: P. Markstein, IBM J. Res. Dev. 34,
+// 1990; J.-M. Muller et al., Handbook of Floating-Point Arithmetic, ch. 4).
+// A quotient q within one ulp of a/b with its exact residual r = a - b q
+// gives fl(q + r y) = the correctly rounded a/b unless the error of r y
+// reaches the distance of a/b from a midpoint of two doubles.  That distance
+// is at least 2^-53/m ulp, m in [1, 2) the significand of b; next to a
+// midpoint |a/b - q| is half an ulp, so |b y - 1| < 2^-52/m is enough.
+// Recip's y is y0 (1 + e + e^2 + e^3), e = 1 - b y0, rounded: |b y - 1| <=
+// m 2^-54 + |e| 2^-53 + e^4 (half an ulp of y, the rounding of the polynomial,
+// its truncation).  With m = 2 (1 - n) both hold where n > |e|/2 + 2^52 e^4.
+// y0 is PTX's rcp.approx.ftz.f64.  Its |e|, a function of the upper significand
+// field but for the exact product, is at most 2^-19.94 over all fields on the
+// B200 and 2^-20.95 where the upper 12 bits are ones.  Guard takes out the
+// denominators whose upper 20 significand bits are ones, n <= 2^-21, and the
+// bound asks for n > 2^-21.95 next to them and n > 2^-20.93 anywhere
+// (tests/f64_seed.cu goes through every field).  18 bits would cover |e| up to
+// 2^-19 at any denominator, but a waiting CTA pays for the fallback: 64^3 59.5
+// -> 61.7 us a stage, 128^3 389.0 -> 391.5.  The first quotient a y is within
+// 1.5 ulp, one residual step makes it faithful, the second correctly rounds it.
 //
-// Measured on the B200 (256^3 ... see the stage kernel's comment).
+// G cell-updates/s a stage of a periodic 192^3 AUSM+ patch on the B200: 2.57
+// with `/`, 4.02 with these quotients, 5.66 with one copy of the face code too
+// (fv_stage_tile).
 #pragma once
 
 #include "fv_numerics.cuh"
 
 namespace dn {
+
+#ifdef __CUDACC__   // (a host test of this arithmetic restates the two instructions)
+// largest of three floats, NaN if any is
+__device__ __forceinline__ float max_nan(float a, float b, float c)
+{
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(a) : "f"(a), "f"(b), "f"(c));
+  return a;
+}
+// approximate reciprocal from the upper 32 bits
+__device__ __forceinline__ double rcp_seed(double b)
+{
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+  return y;
+}
+#endif
 
 // What a thread's fast evaluation must not be trusted for.  The extrema of
 // high words (exponent and upper significand) are accumulated and judged
@@ -55,9 +78,7 @@ struct Guard {
   __device__ __forceinline__ void den(double b) { mant = max(mant, (unsigned)__double2hiint(b) & 0xfffffu); }
   __device__ __forceinline__ void diff(double x, double y)
   {
-    asm("max.NaN.f32 %0, %1, %2, %3;"
-        : "=f"(dmax) : "f"(dmax), "f"(fabsf(__int_as_float(__double2hiint(x)))),
-          "f"(fabsf(__int_as_float(__double2hiint(y)))));
+    dmax = max_nan(dmax, fabsf(__int_as_float(__double2hiint(x))), fabsf(__int_as_float(__double2hiint(y))));
   }
   __device__ __forceinline__ void num(double x) { zmin = min(zmin, ((unsigned)__double2hiint(x) & 0x7fffffffu) - 1u); }
   __device__ __forceinline__ void positive(double x)
@@ -65,21 +86,15 @@ struct Guard {
     lo = min(lo, __double2hiint(x));
     hi = max(hi, __double2hiint(x));
   }
-  // numerators above 2^-500, differences below 2^400 over denominators of at
-  // least 1e-10, positive quantities in [2^-300, 2^300] (NaN is outside)
+  // trusted: denominators whose upper 20 significand bits are not all ones, numerators
+  // above 2^-500, differences below 2^400 over denominators of at least 1e-10,
+  // positive quantities in [2^-300, 2^300] (NaN is outside)
   __device__ __forceinline__ bool any() const
   {
-    return mant == 0xfffffu || !(dmax < __int_as_float(exp_hi(400))) || zmin < (unsigned)exp_hi(-500) || lo < exp_hi(-300) ||
-           hi >= exp_hi(300) || minus_zero;
+    return mant == 0xfffffu || !(dmax < __int_as_float(exp_hi(400))) || zmin < (unsigned)exp_hi(-500) ||
+           lo < exp_hi(-300) || hi >= exp_hi(300) || minus_zero;
   }
 };
-
-__device__ __forceinline__ double rcp_seed(double b)
-{
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-  return y;
-}
 
 // x * 2^n by its exponent field (x normal, result normal)
 __device__ __forceinline__ double scale2(double x, int n)
