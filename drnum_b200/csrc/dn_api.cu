@@ -18,6 +18,7 @@
 #include "fv_batch.cuh"
 #include "fv_schemes.cuh"
 #include "dn_gridio.h"
+#include "dn_range.h"
 #include <nvtx3/nvToolsExt.h>
 
 #include <cmath>
@@ -46,7 +47,7 @@ struct DnPatch {
   int kp = 0;                               // row pitch along k in elements: FX32 nk rounded up to a
                                             // multiple of 4 (16-byte rows for TMA boxes), FP64 nk
   size_t ncp = 0;                           // device elements per variable, ni*nj*kp
-  int i_chunk = 0;                          // FX32 single-patch launch: planes per CTA (0: default)
+  int i_chunk = 0;                          // single-patch launch: planes per CTA (0: not chosen yet)
   void* buf[3] = {nullptr, nullptr, nullptr};
   uint8_t* active = nullptr;
   double base[5] = {0, 0, 0, 0, 0};
@@ -194,18 +195,8 @@ struct dn_ctx {
 
 namespace {
 
-// Planes per CTA of a single-patch launch: the range whose launch takes the
-// least time when a CTA's planes take 1 + share * r each (r CTAs resident on
-// its SM), prolog of them are spent on its prologue, and CTAs beyond a wave
-// wait for it.  Short ranges give a small patch the CTAs to fill the GPU (a
-// CTA's planes are a serial chain), long ones spend less on prologues, and
-// the last wave decides between them.  Fitted to both kernels on eleven
-// patches of 16^3 to 40 x 200 x 200 cells with ranges of 1 to 86 planes: the
-// choice is within 3 % of the best measured range but for two (FP32 40 x 200
-// x 200 22 %, FP64 97 x 61 x 83 8 %).  Against the fixed rule before (about four
-// waves of at least eight planes), us a stage: FP32 16^3 39.0 -> 10.4, 32^3
-// 34.9 -> 10.4, 64^3 32.9 -> 18.6; FP64 16^3 68 -> 14.7, 32^3 70.4 -> 17.5,
-// 64^3 82.3 -> 60.7.
+// Work split of batched stages: CTAs of n planes take n + prolog, slowed by 1 +
+// share * r while r of them share an SM, and CTAs beyond a wave wait for it.
 struct ChunkCost {
   int ctas_per_sm;   // resident CTAs of the kernel
   double prolog;     // prologue in planes
@@ -245,10 +236,20 @@ int best_range(const std::vector<std::pair<int, long>>& runs, int num_sms, const
   return best_ic;
 }
 
-int default_i_chunk(int ni, int nj, int nk, int tj, int tk, int num_sms, const ChunkCost& k)
+// Planes per CTA of a single-patch launch, the `count` predicted fastest.
+std::vector<int> plane_ranges(const dn_ctx* c, const DnPatch& p, size_t count)
 {
-  const long tiles = (long)((nj + tj - 1) / tj) * ((nk + tk - 1) / tk);
-  return best_range({{ni, tiles}}, num_sms, k);
+  int tj = 4, tk = 32;
+  if (c->precision == DN_FP32) dn::fx32_tile(&tj, &tk);
+  return dn::best_ranges(p.d.ni, p.d.nj, p.d.nk, tj, tk, c->num_sms,
+                         c->precision == DN_FP32 ? dn::kRangeFx32 : dn::kRangeF64, count);
+}
+
+// ... the patch's own: predicted once, or tuned
+int plane_range(const dn_ctx* c, DnPatch& p)
+{
+  if (p.i_chunk == 0) p.i_chunk = plane_ranges(c, p, 1)[0];
+  return p.i_chunk;
 }
 
 constexpr int kSumThreads = 256;
@@ -1615,7 +1616,7 @@ int stage_patch(dn_ctx* c, DnPatch& p, int in_b, int un_b, int out_b, double fac
     a.active = p.active;
     a.err = c->d_err;
     a.err_info = c->d_err_info;
-    g.i_chunk = default_i_chunk(g.ni, g.nj, g.nk, 4, 32, c->num_sms, kChunkF64);
+    g.i_chunk = plane_range(c, p);
     a.g = g;
     a.p.Ax = dy * dz; a.p.Ay = dx * dz; a.p.Az = dx * dy; a.p.pf = pf;
     a.wall = p.wall;
@@ -1628,12 +1629,9 @@ int stage_patch(dn_ctx* c, DnPatch& p, int in_b, int un_b, int out_b, double fac
     a.active = p.active;
     a.err = c->d_err;
     a.err_info = c->d_err_info;
-    int tj, tk;
-    dn::fx32_tile(&tj, &tk);
     a.g.ni = g.ni; a.g.nj = g.nj; a.g.nk = g.nk; a.g.kp = p.kp;
     a.g.per_x = g.per_x; a.g.per_y = g.per_y; a.g.per_z = g.per_z;
-    a.g.i_chunk = p.i_chunk > 0 ? std::min(p.i_chunk, g.ni)
-                                : default_i_chunk(g.ni, g.nj, g.nk, tj, tk, c->num_sms, kChunkFx32);
+    a.g.i_chunk = plane_range(c, p);
     dn::fx_set_params(a.p, dx, dy, dz, factor, p.base, p.quantum);
     a.wall = p.wall;
     e = dn::launch_stage_fx32(a, c->stream);
@@ -2012,6 +2010,8 @@ int add_patch(dn_ctx* c, const dn_patch_desc* d, int* id, bool compact)
     cudaMemsetAsync(p.buf[b], 0, bytes, c->stream);
   }
   c->patches.push_back(p);
+  // a lone patch is stepped by single-patch launches (others as far as batching is off)
+  if (c->patches.size() == 1 && !compact) plane_range(c, c->patches[0]);
   c->tables.resize(c->patches.size());
   c->ls.resize(c->patches.size());
   c->ls_on.resize(c->patches.size(), 0);
@@ -3098,9 +3098,7 @@ int dn_autotune(dn_ctx* c, const char* cache_path, double cost_out[DN_NUM_TILE_S
     for (size_t q = 0; q < c->patches.size(); ++q) {
       DnPatch& P = c->patches[q];
       if (!P.owned) continue;
-      int tj, tk;
-      dn::fx32_tile(&tj, &tk);
-      const int def = default_i_chunk(P.d.ni, P.d.nj, P.d.nk, tj, tk, c->num_sms, kChunkFx32);
+      const int def = plane_ranges(c, P, 1)[0];
       const int cand[11] = {def, 8, 12, 16, 20, 24, 28, 32, 40, 48, 64};
       int best = def;
       double best_ms = 1e300;
