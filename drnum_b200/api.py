@@ -536,9 +536,10 @@ class B200CartesianIterator:
         check(self.ctx, self.lib.dn_patch_set_tile(self.ctx, int(i_patch), int(shape)))
 
     def autotune(self, cache_path=None):
-        """Measures the tile shapes on this case and picks one per patch (and,
-        for FP32-bulk single-patch launches, the plane-chunk length of the
-        CTAs); returns the measured cost per padded cell (ns) of each shape."""
+        """Measures the tile shapes on this case and picks one per patch, with
+        the schedule of the batched launches (for single-patch launches the
+        plane-chunk length of the CTAs); returns the measured cost per padded
+        cell (ns) of each shape."""
         cost = np.zeros(_lib.DN_NUM_TILE_SHAPES)
         path = None if cache_path is None else str(cache_path).encode()
         check(self.ctx, self.lib.dn_autotune(self.ctx, path, _lib.dptr(cost)))

@@ -237,12 +237,12 @@ int best_range(const std::vector<std::pair<int, long>>& runs, int num_sms, const
 }
 
 // Planes per CTA of a single-patch launch, the `count` predicted fastest.
-std::vector<int> plane_ranges(const dn_ctx* c, const DnPatch& p, size_t count)
+std::vector<int> plane_ranges(const dn_ctx* c, const DnPatch& p, size_t count, bool every = false)
 {
   int tj = 4, tk = 32;
   if (c->precision == DN_FP32) dn::fx32_tile(&tj, &tk);
   return dn::best_ranges(p.d.ni, p.d.nj, p.d.nk, tj, tk, c->num_sms,
-                         c->precision == DN_FP32 ? dn::kRangeFx32 : dn::kRangeF64, count);
+                         c->precision == DN_FP32 ? dn::kRangeFx32 : dn::kRangeF64, count, every);
 }
 
 // ... the patch's own: predicted once, or tuned
@@ -3087,40 +3087,41 @@ int dn_autotune(dn_ctx* c, const char* cache_path, double cost_out[DN_NUM_TILE_S
     if (s2 != DN_OK) return s2;
     write_tune_cache(cache_path, dev, c->precision, cost);
   }
-  // FX32 stages that run the single-patch kernel (one patch, or batching
-  // off): the plane-chunk length of its CTAs, measured among a few
-  // candidates on the patch itself (one stage into the scratch field,
-  // factor 0; the chunking changes no result)
-  if (c->precision == DN_FP32 && (c->patches.size() == 1 || !c->batched)) {
+  // stages that run the single-patch kernel (one patch, or batching off): the
+  // plane range of its CTAs, measured among a few predicted fastest on the
+  // patch itself (one stage into the scratch field, factor 0; the range changes
+  // no result).  On the 284 patches the prediction was fitted to, the best of
+  // the six (FP64 four: it predicts them better) is within 0.1 % of the fastest
+  // measured range on average and 5 % at most.  Ten fixed ranges of 8 to 64
+  // planes took 256^3 60 ms, now 32, and found 1610 us a step, now 1575.
+  if ((c->patches.size() == 1 || !c->batched) && !functor_stage(c)) {
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    for (size_t q = 0; q < c->patches.size(); ++q) {
-      DnPatch& P = c->patches[q];
+    int st = DN_OK;
+    for (DnPatch& P : c->patches) {
       if (!P.owned) continue;
-      const int def = plane_ranges(c, P, 1)[0];
-      const int cand[11] = {def, 8, 12, 16, 20, 24, 28, 32, 40, 48, 64};
-      int best = def;
+      int best = 0;
       double best_ms = 1e300;
-      for (int k = 0; k < 11; ++k) {
-        if (cand[k] > P.d.ni || (k > 0 && cand[k] == def)) continue;
-        P.i_chunk = cand[k];
-        int st = DN_OK;
-        for (int r = 0; r < 7 && st == DN_OK; ++r) {
-          if (r == 2) cudaEventRecord(e0, c->stream);
+      for (int range : plane_ranges(c, P, c->precision == DN_FP32 ? 6 : 4, true)) {
+        P.i_chunk = range;
+        for (int r = 0; r < 4 && st == DN_OK; ++r) {
+          if (r == 1) cudaEventRecord(e0, c->stream);
           st = stage_patch(c, P, c->fmap[0], c->fmap[1], c->fmap[2], 0.0);
         }
+        if (st != DN_OK) break;
         cudaEventRecord(e1, c->stream);
         cudaEventSynchronize(e1);
-        if (st != DN_OK) { P.i_chunk = 0; cudaEventDestroy(e0); cudaEventDestroy(e1); return st; }
         float ms = 0;
         cudaEventElapsedTime(&ms, e0, e1);
-        if (ms < best_ms) { best_ms = ms; best = cand[k]; }
+        if (ms < best_ms) { best_ms = ms; best = range; }
       }
       P.i_chunk = best;
+      if (st != DN_OK) break;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    if (st != DN_OK) return st;
     int s3 = read_device_error(c);
     if (s3 != DN_OK) return s3;
   }
@@ -3135,75 +3136,72 @@ int dn_autotune(dn_ctx* c, const char* cache_path, double cost_out[DN_NUM_TILE_S
   }
   c->batch_dirty = true;
   c->generation++;
-  // batched stages: the schedule of the work items, measured among a few
-  // candidates with the shapes just chosen (one stage of every patch into
-  // the scratch field, factor 0; the schedule changes no result): FP64 the
-  // shortest plane range of an item; FX32 that, or instead the waves of
-  // persistent CTAs (fewer waves save prologues, more let the hardware even
-  // out tiles of unequal cost, one CTA per item keeps neighbouring columns
-  // on the same planes at the same time)
+  // batched stages: tile shapes and the schedule of the work items together
+  // (one stage of every patch into the scratch field, factor 0; they change no
+  // result): FP64 the shortest plane range of an item, or the ranges of the cost
+  // model; FX32 the waves of persistent CTAs (fewer waves save prologues, more
+  // let the hardware even out tiles of unequal cost) or one CTA per item (it
+  // keeps neighbouring columns on the same planes at the same time).  The costs
+  // were measured with one schedule, and neither choice is best without the
+  // other (level-set sphere 732 us a step when the schedule was tuned for the
+  // per-patch shapes only, 699 with 16 x 32 tiles in one wave).  So the shapes
+  // chosen per patch and each shape for all patches are tried with the schedule
+  // that is fastest or nearly so on most grids, then the other schedules with
+  // the fastest of those: eight trials at most.  (Fifteen trials that left out
+  // uniform shapes and the 24-plane schedule took longer, 64 uneven patches 74 ms
+  // against 43, and found slower pairs, us a step: jet 1546 against 1482, at 0.7
+  // of its size 826 against 751, 64 uneven patches at 0.8 960 against 851.)
   if (c->batched && c->patches.size() > 1) {
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     const bool fp64 = c->precision == DN_FP64;
     // (waves, shortest item): persistent waves for FP32 bulk, or one CTA per
-    // item; 0, 0: FP64 ranges by the cost model
-    const int cand64[4][2] = {{0, 0}, {0, 8}, {0, 16}, {0, 32}};
-    const int cand32[5][2] = {{1, 8}, {2, 8}, {4, 8}, {0, 8}, {0, 16}};
-    const int n_cand = fp64 ? 4 : 5;
-    // with the shapes chosen per patch, and with the one shape that is
-    // fastest for all of them: the costs were measured with one schedule, and
-    // shapes and schedule together decide (level-set sphere 732 us a step
-    // when the schedule was tuned for the per-patch shapes only, 699 with
-    // 16 x 32 tiles in one wave)
+    // item; 0, 0: FP64 ranges by the cost model.  Of 20 workloads (jet, sphere
+    // and uneven grids of several scales) the first was the fastest of all
+    // schedules but on two; one CTA per 24 planes took the full-size jet from
+    // 477 to 454 us a stage, one per 8 planes a grid of few patches from 131 to
+    // 121.
+    const int cand64[3][2] = {{0, 0}, {0, 8}, {0, 16}};
+    const int cand32[5][2] = {{1, 8}, {2, 8}, {0, 8}, {0, 16}, {0, 24}};
+    const int (*cand)[2] = fp64 ? cand64 : cand32;
+    const int n_cand = fp64 ? 3 : 5;
     std::vector<std::vector<int>> shapes(1, c->shape);
-    {
-      int u = 0;
-      double best_u = 1e300;
-      for (int sh = 0; sh < dn::kNumShapes; ++sh) {
-        double t = 0;
-        for (size_t q = 0; q < c->patches.size(); ++q)
-          if (c->patches[q].owned) t += cost[sh] * padded_cells(c, c->patches[q], sh);
-        if (t < best_u) { best_u = t; u = sh; }
-      }
-      for (int sh = 0; sh < dn::kNumShapes; ++sh) {
-        // 16 x 32 tiles too (FP32): fewest halo cells
-        if (sh != u && (fp64 || sh != 2)) continue;
-        std::vector<int> all(c->shape.size(), sh);
-        if (std::find(shapes.begin(), shapes.end(), all) == shapes.end()) shapes.push_back(all);
-      }
+    for (int sh = 0; sh < dn::kNumShapes; ++sh) {
+      std::vector<int> all(c->shape.size(), sh);
+      if (all != c->shape) shapes.push_back(all);
     }
     std::vector<int> best_s = c->shape;
     int best_w = c->batch_waves, best_p = c->batch_min_planes;
     bool best_a = c->batch_auto;
     double best_ms = 1e300;
     int st = DN_OK;
-    for (size_t m = 0; m < shapes.size() && st == DN_OK; ++m) {
-      for (int k = 0; k < n_cand && st == DN_OK; ++k) {
-        c->shape = shapes[m];
-        c->batch_waves = fp64 ? cand64[k][0] : cand32[k][0];
-        const int mp = fp64 ? cand64[k][1] : cand32[k][1];
-        c->batch_auto = mp == 0;
-        c->batch_min_planes = mp ? mp : 8;
-        c->batch_dirty = true;
-        for (int r = 0; r < 5 && st == DN_OK; ++r) {
-          if (r == 2) cudaEventRecord(e0, c->stream);
-          st = stage_all(c, c->fmap[0], c->fmap[1], c->fmap[2], 0.0);
-        }
-        cudaEventRecord(e1, c->stream);
-        cudaEventSynchronize(e1);
-        float ms = 0;
-        cudaEventElapsedTime(&ms, e0, e1);
-        if (st == DN_OK && ms < best_ms) {
-          best_ms = ms;
-          best_s = c->shape;
-          best_w = c->batch_waves;
-          best_p = c->batch_min_planes;
-          best_a = c->batch_auto;
-        }
+    auto trial = [&](const std::vector<int>& shape, const int k[2]) {
+      c->shape = shape;
+      c->batch_waves = k[0];
+      c->batch_auto = k[1] == 0;
+      c->batch_min_planes = k[1] ? k[1] : 8;
+      c->batch_dirty = true;
+      for (int r = 0; r < 5 && st == DN_OK; ++r) {
+        if (r == 2) cudaEventRecord(e0, c->stream);
+        st = stage_all(c, c->fmap[0], c->fmap[1], c->fmap[2], 0.0);
       }
-    }
+      if (st != DN_OK) return;
+      cudaEventRecord(e1, c->stream);
+      cudaEventSynchronize(e1);
+      float ms = 0;
+      cudaEventElapsedTime(&ms, e0, e1);
+      if (ms < best_ms) {
+        best_ms = ms;
+        best_s = c->shape;
+        best_w = c->batch_waves;
+        best_p = c->batch_min_planes;
+        best_a = c->batch_auto;
+      }
+    };
+    for (size_t m = 0; m < shapes.size() && st == DN_OK; ++m) trial(shapes[m], cand[0]);
+    const std::vector<int> shape = best_s;
+    for (int k = 1; k < n_cand && st == DN_OK; ++k) trial(shape, cand[k]);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     c->shape = best_s;

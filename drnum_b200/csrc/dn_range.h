@@ -106,8 +106,9 @@ struct RangeLaunch {
 };
 
 // The `count` fastest ranges, fastest first, of the shortest ranges of every
-// number of CTAs along i (65535 at most: the grid's third extent); of those the
-// count + 7 with the lowest bounds are simulated (under 1 ms).
+// number of CTAs along i (65535 at most: the grid's third extent), or of `every`
+// range up to 64 planes; of those the count + 7 with the lowest bounds are
+// simulated (1 ms, 2 ms with every range).
 //
 // A CTA's planes are a serial chain: short ranges give a small patch the CTAs
 // to fill the GPU, long ones spend less on prologues, and the last CTAs decide
@@ -121,7 +122,8 @@ struct RangeLaunch {
 // Whole waves of equal CTAs in place of the simulation chose 121 us for FP64 97
 // x 61 x 83, whose last row of tiles has one row of four, where eight planes
 // take 109, and 99 against 94 for FP32 45 x 198 x 167.
-inline std::vector<int> best_ranges(int ni, int nj, int nk, int tj, int tk, int sms, const RangeCost& c, size_t count)
+inline std::vector<int> best_ranges(int ni, int nj, int nk, int tj, int tk, int sms, const RangeCost& c, size_t count,
+                                    bool every = false)
 {
   std::vector<RangeLaunch> launches;
   for (int chunks = 1; chunks <= std::min(ni, 65535);) {
@@ -129,10 +131,12 @@ inline std::vector<int> best_ranges(int ni, int nj, int nk, int tj, int tk, int 
     launches.emplace_back(ni, nj, nk, tj, tk, ic, sms, c);
     if (ic == 1) break;
     chunks = (ni + ic - 2) / (ic - 1);   // the fewest with a shorter range
+    for (int q = std::min(ic - 1, 64); every && q > (ni + chunks - 1) / chunks; --q)
+      launches.emplace_back(ni, nj, nk, tj, tk, q, sms, c);
   }
   std::sort(launches.begin(), launches.end(),
             [](const RangeLaunch& a, const RangeLaunch& b) { return a.lower_bound() < b.lower_bound(); });
-  launches.erase(launches.begin() + (long)std::min(launches.size(), count + 7), launches.end());
+  launches.erase(launches.begin() + (long)std::min(launches.size(), 4 * count + 4), launches.end());
   std::vector<std::pair<double, int>> best;
   for (const RangeLaunch& l : launches) {
     const double limit = best.size() < count ? 1e300 : best.back().first;

@@ -1,0 +1,56 @@
+"""What the autotuner spends and what it changes, with given tile shape costs (a
+cache file), so that nothing of its trials depends on a clock."""
+import numpy as np
+import pytest
+
+from drnum_b200 import cases
+from drnum_b200._lib import DN_FP32, DN_FP64
+from drnum_b200.api import AusmPlus, B200CartesianIterator, CartesianPatch
+
+pytestmark = pytest.mark.gpu
+
+
+def iterator(extents, precision):
+    it = B200CartesianIterator(AusmPlus(), 0, precision)
+    for n in extents:
+        p = CartesianPatch(*n, spacing=(0.1,) * 3, periodic=(True,) * 3)
+        p.setField(0, cases.random_state(*n, seed=1, amp=0.01, mach=0.2))
+        it.addPatch(p)
+    it.updateDevice(fields=(0,))
+    return it
+
+
+@pytest.fixture
+def equal_costs(tmp_path):
+    """A cache file with the same cost for every tile shape."""
+    def make(precision):
+        path = tmp_path / "tune.txt"
+        it = iterator([(8, 8, 32), (8, 8, 32)], precision)
+        cost = it.autotune(path)
+        it.close()
+        line = path.read_text().strip().split("|")
+        path.write_text("|".join(line[:-len(cost)] + ["1"] * len(cost)) + "\n")
+        return path
+    return make
+
+
+def test_trials_of_a_grid(equal_costs):
+    # an 8 x 32 and a 16 x 16 cross-section: per-patch shapes differ, so every
+    # uniform shape is tried as well; eight trials of five stages, two launches each
+    path = equal_costs(DN_FP32)
+    it = iterator([(16, 8, 32), (16, 16, 16)], DN_FP32)
+    before = it.launchCount()
+    assert np.array_equal(it.autotune(path), np.ones(3))
+    assert 0 < it.launchCount() - before <= 8 * 5 * 2
+    it.close()
+
+
+@pytest.mark.parametrize("precision", [DN_FP64, DN_FP32])
+def test_trials_of_a_patch(equal_costs, precision):
+    # a lone patch: its plane ranges, six of seven stages at most
+    path = equal_costs(precision)
+    it = iterator([(64, 32, 32)], precision)
+    before = it.launchCount()
+    assert np.array_equal(it.autotune(path), np.ones(3))
+    assert 0 < it.launchCount() - before <= 6 * 7
+    it.close()
