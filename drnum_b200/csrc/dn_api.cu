@@ -158,7 +158,7 @@ struct dn_ctx {
   // deals the work to that many waves of persistent CTAs; 0 launches one
   // CTA per work item, items of at least batch_min_planes planes
   int batch_min_planes = 8;
-  bool batch_auto = true;   // FP64: plane ranges by the cost model until a shortest range is set
+  bool batch_auto = true;   // FP64: plane ranges by the cost model instead
   int batch_waves = 2;
   cudaStream_t s_aux = nullptr;               // second branch of a batched stage (inside and edge tiles)
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -2680,7 +2680,7 @@ int dn_set_option(dn_ctx* c, int option, int value)
     if (value < (option == DN_OPT_BATCH_WAVES ? 0 : 1) || value > 64)
       return fail(c, DN_ERR_ARG, "schedule option %d out of range: %d", option, value);
     (option == DN_OPT_BATCH_WAVES ? c->batch_waves : c->batch_min_planes) = value;
-    if (option == DN_OPT_BATCH_MIN_PLANES) c->batch_auto = false;
+    if (option == DN_OPT_BATCH_MIN_PLANES) c->batch_auto = value == 8;   // the default is the model's ranges
     c->batch_dirty = true;
     c->generation++;
     return DN_OK;

@@ -363,8 +363,8 @@ int dn_lslayers_destroy(dn_lslayers* ls);
  *     work to that many waves of persistent CTAs with equal planes per CTA;
  *     0 launches one CTA per work item.  dn_autotune measures the choices.
  *   DN_OPT_BATCH_MIN_PLANES (default 8): shortest plane range of a work item
- *     when one CTA takes one item.  FP64 launches take the range a cost model
- *     predicts fastest until this is set (or tuned).
+ *     when one CTA takes one item.  With the default FP64 launches take the
+ *     range a cost model predicts fastest instead (so does setting 8 again).
  *   DN_OPT_DONOR_TABLES (default 0): device form of the donor tables.  0 =
  *     interpolation patterns (each group as donor patch, first donor cell and
  *     a shared entry of offsets and weights) wherever every device cell

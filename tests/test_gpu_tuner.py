@@ -1,10 +1,12 @@
 """What the autotuner spends and what it changes, with given tile shape costs (a
 cache file), so that nothing of its trials depends on a clock."""
+import time
+
 import numpy as np
 import pytest
 
 from drnum_b200 import cases
-from drnum_b200._lib import DN_FP32, DN_FP64
+from drnum_b200._lib import DN_FP32, DN_FP64, DN_OPT_BATCH_MIN_PLANES
 from drnum_b200.api import AusmPlus, B200CartesianIterator, CartesianPatch
 
 pytestmark = pytest.mark.gpu
@@ -53,4 +55,27 @@ def test_trials_of_a_patch(equal_costs, precision):
     before = it.launchCount()
     assert np.array_equal(it.autotune(path), np.ones(3))
     assert 0 < it.launchCount() - before <= 6 * 7
+    it.close()
+
+
+def test_default_range_comes_back():
+    # FP64 patches of few columns: the default takes ranges of a plane or two,
+    # 32 planes are many times slower, and setting the default again is the default
+    it = iterator([(64, 16, 32), (64, 16, 32)], DN_FP64)
+
+    def step():
+        best = 1e9
+        for _ in range(20):
+            it.sync()
+            t = time.perf_counter()
+            it.rkStep(1e-9, cases.RK3_ALPHA)
+            it.sync()
+            best = min(best, time.perf_counter() - t)
+        return best
+
+    default = step()
+    it.setOption(DN_OPT_BATCH_MIN_PLANES, 32)
+    assert step() > 3 * default
+    it.setOption(DN_OPT_BATCH_MIN_PLANES, 8)
+    assert step() < 1.5 * default
     it.close()
