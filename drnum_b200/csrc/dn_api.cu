@@ -2996,8 +2996,12 @@ std::string device_name(int dev)
   return prop.name;
 }
 
-// cache lines: "<device>|<precision>|<shapes>|<cost shape 0>|<cost shape 1>|..."
-bool read_tune_cache(const char* path, const std::string& dev, int precision, double cost[dn::kNumShapes])
+// cache lines: "<device>|<precision>|<scheme>.<revision>|<shapes>|<cost shape 0>|<cost shape 1>|..."
+// Schemes differ in cost per padded cell; the revision goes up when a change of
+// the stage kernels or of their default schedule makes older costs wrong.
+constexpr int kTuneRevision = 1;
+
+bool read_tune_cache(const char* path, const std::string& dev, int precision, int scheme, double cost[dn::kNumShapes])
 {
   if (!path) return false;
   FILE* f = std::fopen(path, "r");
@@ -3006,9 +3010,9 @@ bool read_tune_cache(const char* path, const std::string& dev, int precision, do
   bool found = false;
   while (std::fgets(line, sizeof line, f)) {
     char name[256];
-    int prec, ns, pos = 0;
-    if (std::sscanf(line, "%255[^|]|%d|%d%n", name, &prec, &ns, &pos) != 3 || dev != name || prec != precision ||
-        ns != dn::kNumShapes)
+    int prec, sch, rev, ns, pos = 0;
+    if (std::sscanf(line, "%255[^|]|%d|%d.%d|%d%n", name, &prec, &sch, &rev, &ns, &pos) != 5 || dev != name ||
+        prec != precision || sch != scheme || rev != kTuneRevision || ns != dn::kNumShapes)
       continue;
     double c[dn::kNumShapes];
     const char* q = line + pos;
@@ -3027,12 +3031,13 @@ bool read_tune_cache(const char* path, const std::string& dev, int precision, do
   return found;
 }
 
-void write_tune_cache(const char* path, const std::string& dev, int precision, const double cost[dn::kNumShapes])
+void write_tune_cache(const char* path, const std::string& dev, int precision, int scheme,
+                      const double cost[dn::kNumShapes])
 {
   if (!path) return;
   FILE* f = std::fopen(path, "a");
   if (!f) return;
-  std::fprintf(f, "%s|%d|%d", dev.c_str(), precision, dn::kNumShapes);
+  std::fprintf(f, "%s|%d|%d.%d|%d", dev.c_str(), precision, scheme, kTuneRevision, dn::kNumShapes);
   for (int k = 0; k < dn::kNumShapes; ++k) std::fprintf(f, "|%.17g", cost[k]);
   std::fprintf(f, "\n");
   std::fclose(f);
@@ -3050,7 +3055,8 @@ int dn_autotune(dn_ctx* c, const char* cache_path, double cost_out[DN_NUM_TILE_S
   const std::string dev = device_name(c->device);
   static_assert(DN_NUM_TILE_SHAPES == dn::kNumShapes, "tile shape count");
   double cost[dn::kNumShapes] = {};
-  if (!read_tune_cache(cache_path, dev, c->precision, cost)) {
+  const int scheme = functor_stage(c) ? DN_FLUX_AUSMPLUS_FUNCTOR : c->scheme;
+  if (!read_tune_cache(cache_path, dev, c->precision, scheme, cost)) {
     // measure each tile shape on the case itself: one stage of every patch
     // into the scratch field (field 2), factor 0
     const std::vector<int> saved = c->shape;
@@ -3085,7 +3091,7 @@ int dn_autotune(dn_ctx* c, const char* cache_path, double cost_out[DN_NUM_TILE_S
     if (st != DN_OK) { c->batch_dirty = true; c->generation++; return st; }
     int s2 = read_device_error(c);
     if (s2 != DN_OK) return s2;
-    write_tune_cache(cache_path, dev, c->precision, cost);
+    write_tune_cache(cache_path, dev, c->precision, scheme, cost);
   }
   // stages that run the single-patch kernel (one patch, or batching off): the
   // plane range of its CTAs, measured among a few predicted fastest on the

@@ -390,8 +390,9 @@ int dn_patch_set_tile(dn_ctx* ctx, int patch_id, int shape);
 /* Autotuner: measures each tile shape's cost per padded cell on the
  * context's own patches (one stage into the scratch field 2, which it
  * overwrites), then gives every patch the shape of least predicted time.
- * cache_path (may be NULL) holds measured costs per device and precision and
- * is reused on the next call; cost_out[DN_NUM_TILE_SHAPES] (may be NULL) returns them in ns per
+ * cache_path (may be NULL) holds measured costs per device, precision and flux
+ * scheme and is reused on the next call (lines of other libraries are left
+ * alone); cost_out[DN_NUM_TILE_SHAPES] (may be NULL) returns them in ns per
  * padded cell and stage.  Stages that run one patch per launch (a single
  * patch, or batching off; not those of a functor) also get the plane-chunk
  * length of their CTAs, measured among a few candidates on the patch itself;

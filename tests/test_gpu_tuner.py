@@ -7,13 +7,13 @@ import pytest
 
 from drnum_b200 import cases
 from drnum_b200._lib import DN_FP32, DN_FP64, DN_OPT_BATCH_MIN_PLANES
-from drnum_b200.api import AusmPlus, B200CartesianIterator, CartesianPatch
+from drnum_b200.api import AusmPlus, B200CartesianIterator, CartesianPatch, Roe, VanLeer
 
 pytestmark = pytest.mark.gpu
 
 
-def iterator(extents, precision):
-    it = B200CartesianIterator(AusmPlus(), 0, precision)
+def iterator(extents, precision, scheme=AusmPlus):
+    it = B200CartesianIterator(scheme(), 0, precision)
     for n in extents:
         p = CartesianPatch(*n, spacing=(0.1,) * 3, periodic=(True,) * 3)
         p.setField(0, cases.random_state(*n, seed=1, amp=0.01, mach=0.2))
@@ -79,3 +79,22 @@ def test_default_range_comes_back():
     it.setOption(DN_OPT_BATCH_MIN_PLANES, 8)
     assert step() < 1.5 * default
     it.close()
+
+
+def test_cache_keeps_schemes_apart(tmp_path):
+    # each scheme reads its own costs, none those of another or of a line without a scheme
+    path = tmp_path / "tune.txt"
+    costs = {}
+    for scheme in (AusmPlus, VanLeer, Roe):
+        it = iterator([(16, 8, 32), (16, 16, 16)], DN_FP64, scheme)
+        costs[scheme] = it.autotune(path)
+        it.close()
+    lines = path.read_text().splitlines()
+    assert len(lines) == 3
+    device, precision = lines[0].split("|")[:2]
+    path.write_text("%s|%s|3|1|1|1\n" % (device, precision) + "\n".join(lines) + "\n")
+    for scheme, cost in costs.items():
+        it = iterator([(16, 8, 32), (16, 16, 16)], DN_FP64, scheme)
+        assert np.array_equal(it.autotune(path), cost)
+        it.close()
+    assert len(path.read_text().splitlines()) == 4
