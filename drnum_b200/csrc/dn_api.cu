@@ -1615,7 +1615,6 @@ int stage_patch(dn_ctx* c, DnPatch& p, int in_b, int un_b, int out_b, double fac
     a.out = (double*)p.buf[out_b];
     a.active = p.active;
     a.err = c->d_err;
-    a.err_info = c->d_err_info;
     g.i_chunk = plane_range(c, p);
     a.g = g;
     a.p.Ax = dy * dz; a.p.Ay = dx * dz; a.p.Az = dx * dy; a.p.pf = pf;

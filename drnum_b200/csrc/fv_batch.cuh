@@ -162,7 +162,6 @@ fv_stage_batched_f64(const Batch b)
     args.out = static_cast<double*>(rec.buf[b.out_b]);
     args.active = rec.active;
     args.err = b.err;
-    args.err_info = b.err_info;
     args.g.ni = rec.ni; args.g.nj = rec.nj; args.g.nk = rec.nk;
     args.g.per_x = rec.per_x; args.g.per_y = rec.per_y; args.g.per_z = rec.per_z;
     args.g.i_chunk = w.i1 - w.i0;

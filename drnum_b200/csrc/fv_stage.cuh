@@ -23,12 +23,9 @@
 //   - the update is written once; inactive cells copy their input
 //     (cartesianiterator.h:315, gpu_cartesianiterator.h:199-201).
 //
-// The storage/arithmetic form is a policy:
-//   Policy::Store   element type in HBM
-//   Policy::Real    arithmetic type
-//   Policy::load(v, x)           stored value -> arithmetic value
-//   Policy::face(v, F)           face flux -> value summed into the residual
-//   Policy::update(v, un, r)     new stored value from stored f_n and residual
+// The storage form is a policy (fv_policies.cuh): its 8-byte values are staged
+// and computed with as they are, and Policy::update(un, r) makes the new value
+// from f_n and the residual.
 #pragma once
 
 #include <cstdint>
@@ -51,8 +48,7 @@ struct StageArgs {
   const typename Policy::Store* un;   // step-start state f(n), own cell only
   typename Policy::Store* out;        // f(k)
   const uint8_t* active;              // per cell, NULL = all active
-  int* err;                           // device error word (bit flags)
-  unsigned long long* err_info;       // first failing cell: [cell, var, bits(un), bits(r)]
+  int* err;                           // device error word (bit flags; here 32, a plane load that did not arrive)
   StageGeom g;
   typename Policy::Params p;
   WallBC wall;                        // patch-face fluxes of the non-periodic axes
@@ -85,13 +81,12 @@ __device__ __forceinline__ bool cell_ok(int x, int n, int per)
 template <class Policy, int TJ, int TK>
 struct StageSmem {
   using Real = typename Policy::Real;
-  using FaceT = typename Policy::FaceT;
   static constexpr int PJ = TJ + 4;
   static constexpr int PK = TK + 4;
   alignas(128) Real plane[3][5][PJ][PK];   // planes i .. i+2
   Real xm[5][TJ * TK];                     // own column of plane i-1 (each thread its own cell)
-  FaceT fy[5][TJ + 1][TK];
-  FaceT fz[5][TJ][TK + 1];
+  Real fy[5][TJ + 1][TK];
+  Real fz[5][TJ][TK + 1];
   alignas(8) uint64_t bar;                 // mbarrier of the TMA plane loads
 };
 
@@ -308,7 +303,6 @@ __device__ __forceinline__ void fv_stage_tile(const StageArgs<Policy>& a, const 
     if (!first && own) {
       const size_t c = (size_t)i * njk + (size_t)j * g.nk + k;
       const bool act = a.active ? (a.active[c] != 0) : true;
-      int bad = 0;
       Real res[5];
       #pragma unroll
       for (int v = 0; v < 5; ++v) {
@@ -325,13 +319,13 @@ __device__ __forceinline__ void fv_stage_tile(const StageArgs<Policy>& a, const 
         #pragma unroll
         for (int v = 0; v < 5; ++v) U[v] = ring[s0 * SS + v * VS + me];
         add_wall_fluxes(a.wall, g.ni, g.nj, g.nk, g.per_x, g.per_y, g.per_z, i, j, k, U, a.p.Ax, a.p.Ay, a.p.Az, res,
-                        [&](int v, Real x) { return Policy::face(a.p, v, x); });
+                        [](int, Real x) { return x; });
       }
       #pragma unroll
       for (int v = 0; v < 5; ++v) {
         typename Policy::Store o;
         if (act) {
-          o = Policy::update(a.p, v, a.un[v * nc + c], res[v], bad);
+          o = Policy::update(a.p, a.un[v * nc + c], res[v]);
         } else {
           o = a.in[v * nc + c];
         }
