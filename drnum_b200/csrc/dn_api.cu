@@ -1233,14 +1233,14 @@ int default_shape(const DnPatch& p)
 // `slots` CTAs (one wave) so that every CTA gets about the same number of
 // planes, each item charged kProlog planes for its prologue (three planes
 // staged and dequantised before the first update).  A CTA's items follow
-// one another along the runs; no piece is shorter than kMinPiece planes
+// one another along the runs; no piece is shorter than `piece` planes
 // where its run is longer.  The share per CTA starts at the even split and
 // grows by 1 % until the deal fits the wave.  Returns the items and the
 // group offsets (groups.size() - 1 CTAs).
 constexpr double kProlog = 3.0;
 constexpr int kMinPiece = 4;
 
-void deal_greedy(const std::vector<dn::WorkItem>& runs, double target, int kMinPiece, std::vector<dn::WorkItem>& items,
+void deal_greedy(const std::vector<dn::WorkItem>& runs, double target, int piece, std::vector<dn::WorkItem>& items,
                  std::vector<int>& groups)
 {
   items.clear();
@@ -1249,14 +1249,14 @@ void deal_greedy(const std::vector<dn::WorkItem>& runs, double target, int kMinP
   for (const auto& r : runs) {
     int i = r.i0;
     while (i < r.i1) {
-      if (acc > 0 && acc + kProlog + kMinPiece > target) {   // this CTA is full
+      if (acc > 0 && acc + kProlog + piece > target) {   // this CTA is full
         groups.push_back((int)items.size());
         acc = 0;
       }
       acc += kProlog;
-      int take = std::max((int)std::ceil(target - acc), kMinPiece);
+      int take = std::max((int)std::ceil(target - acc), piece);
       take = std::min(take, r.i1 - i);
-      if (r.i1 - i - take > 0 && r.i1 - i - take < kMinPiece) take = r.i1 - i;   // no short leftover
+      if (r.i1 - i - take > 0 && r.i1 - i - take < piece) take = r.i1 - i;   // no short leftover
       items.push_back(dn::WorkItem{r.patch, r.j0, r.k0, i, i + take});
       acc += take;
       i += take;
@@ -1265,7 +1265,8 @@ void deal_greedy(const std::vector<dn::WorkItem>& runs, double target, int kMinP
   groups.push_back((int)items.size());
 }
 
-// Too few planes for that (under 2 kMinPiece a CTA): the number of CTAs, in
+// Pieces of kMinPiece planes at least.  Too few planes for that (under 2
+// kMinPiece a CTA): the number of CTAs, in
 // whole CTAs per SM, that the cost model of single-patch launches predicts
 // fastest, down to pieces of a plane.  (A 66 x 64 x 64 sphere pair ran 82 and
 // 50 CTAs of eight planes on 148 SMs.)
@@ -1336,7 +1337,8 @@ void patch_tiles(const dn_ctx* c, const DnPatch& P, int shape, std::vector<TileR
 // Patch records and work items (patch, column tile, plane range) of every
 // patch, grouped by tile form and shape.  FX32: each launch is one wave of
 // persistent CTAs over balanced groups of items (deal_runs).  FP64: plane
-// ranges sized so that the launch holds about four waves of CTAs.
+// ranges of the cost model, or with a set shortest range about four waves of
+// CTAs of at least that (so FP32 without persistent CTAs).
 int build_batch(dn_ctx* c)
 {
   free_batch(c);
