@@ -261,68 +261,25 @@ __device__ __forceinline__ int fx_quant1(float x, FaceRange& r)
 }
 
 // Patch-face flux of side `side` (axis side/2) of a boundary cell with FP32
-// state U, in whole quanta (0 for a zero-flux side), recorded in r: the
-// operations of wall_flux<axis> with the axis chosen at run time.  One copy
-// of this code per call site, in loops that are not unrolled: a copy per
-// axis, side and cell of a pair (twelve in the residual of an edge tile)
-// filled the instruction cache (the single-patch kernel waited for
-// instructions: no_instruction 4.4 of 11.6 warps per issue on a closed 125 x
-// 67 x 93 patch) and spilled (inside form of 16 x 32 tiles 268 bytes a
-// thread, now 72).  Measured together with every side in the slot of the
-// missing face: closed 125 x 67 x 93 patch 79 -> 69 us a stage, 160^3 233 ->
-// 197; RK steps of the jet 1588 -> 1548 us, sphere 704 -> 691, 64 uneven
+// state U, in whole quanta (0 for a zero-flux side), recorded in r.  The axis
+// is chosen at run time, one copy of this code per call site, in loops that
+// are not unrolled: a copy per axis, side and cell of a pair (twelve in the
+// residual of an edge tile) filled the instruction cache (the single-patch
+// kernel waited for instructions: no_instruction 4.4 of 11.6 warps per issue on
+// a closed 125 x 67 x 93 patch) and spilled (inside form of 16 x 32 tiles 268
+// bytes a thread, now 72).  Measured together with every side in the slot of
+// the missing face: closed 125 x 67 x 93 patch 79 -> 69 us a stage, 160^3 233
+// -> 197; RK steps of the jet 1588 -> 1548 us, sphere 704 -> 691, 64 uneven
 // patches 1988 -> 1890.
 __device__ __forceinline__ void fx_wall_quanta(const WallBC& bc, int side, int face, const float U[5], float A,
                                                const float2* face_scale, FaceRange& r, int q[5])
 {
-  const int axis = side >> 1, kind = bc.kind[side];
-  if (kind == kWallZero) {
+  float F[5];
+  if (!wall_flux(bc, side >> 1, side, face, U, A, F)) {
     #pragma unroll
     for (int v = 0; v < 5; ++v) q[v] = 0;
     return;
   }
-  float p1, T1, u1, v1, w1;
-  wall_prim(U, p1, T1, u1, v1, w1);
-  float F[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-  float p = p1;
-  if (kind != kWallSlip) {
-    float Tt = T1, u = u1, v = v1, w = w1;
-    if (kind == kWallInflow) {
-      const double* e = bc.table[side] + (size_t)face * 5;
-      if (e[0] == e[0]) p = (float)e[0];         // NaN: pressure of the boundary cell
-      Tt = (float)e[1];
-      u = (float)e[2];
-      v = (float)e[3];
-      w = (float)e[4];
-    } else {
-      const double* f = bc.ff[side];
-      const float u0 = (float)f[2], v0 = (float)f[3], w0 = (float)f[4], a0 = (float)f[5];
-      const float a1 = sqrtf(float(Gas::gamma) * float(Gas::R) * T1);
-      float M0 = (axis == 0 ? u0 : (axis == 1 ? v0 : w0)) / a0;
-      float M1 = (axis == 0 ? u1 : (axis == 1 ? v1 : w1)) / a1;
-      if (side & 1) {
-        M0 = -M0;
-        M1 = -M1;
-      }
-      const float M = 0.5f * (M0 + M1);
-      if (M >= 0.0f) {
-        if (M >= 1.0f) p = (float)f[0];
-        Tt = (float)f[1];
-        u = u0;
-        v = v0;
-        w = w0;
-      }
-    }
-    F[0] = A * p / (float(Gas::R) * Tt) * (axis == 0 ? u : (axis == 1 ? v : w));
-    F[1] = F[0] * u;
-    F[2] = F[0] * v;
-    F[3] = F[0] * w;
-    F[4] = F[0] * (float(kGasCp) * Tt + 0.5f * (u * u + v * v + w * w));
-  }
-  const float Ap = A * p;
-  F[1] = axis == 0 ? F[1] + Ap : F[1];
-  F[2] = axis == 1 ? F[2] + Ap : F[2];
-  F[3] = axis == 2 ? F[3] + Ap : F[3];
   #pragma unroll
   for (int v = 0; v < 5; ++v) q[v] = fx_quant1(F[v] * face_scale[v].x, r);
 }

@@ -335,7 +335,7 @@ struct SchemeFlux {
   {
     double U[5], F[5];
     p->getVar(0, ic, jc, kc, U);
-    if (wall_flux<AXIS>(wall, s, face, U, A, F))
+    if (wall_flux(wall, AXIS, s, face, U, A, F))
       for (int v = 0; v < 5; ++v) f[v] += F[v];
   }
   template <class P> __device__ void xWallM(P* p, size_t i, size_t j, size_t k, double, double, double, double A, double* f) const

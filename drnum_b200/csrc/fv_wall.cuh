@@ -48,63 +48,61 @@ __device__ __forceinline__ void wall_prim(const T U[5], T& p, T& Tt, T& u, T& v,
   p = U[0] * T(Gas::R) * Tt;
 }
 
-// Flux through a face of axis AXIS from the face state (p, T, u, v, w): the
-// common tail of CompressibleFarfieldFlux and JetFlux::xWallM.
-template <int AXIS, typename T>
-__device__ __forceinline__ void wall_state_flux(T A, T p, T Tt, T u, T v, T w, T F[5])
-{
-  const T un = AXIS == 0 ? u : (AXIS == 1 ? v : w);
-  F[0] = A * p / (T(Gas::R) * Tt) * un;
-  F[1] = F[0] * u;
-  F[2] = F[0] * v;
-  F[3] = F[0] * w;
-  if (AXIS == 0) F[1] = F[1] + A * p;
-  if (AXIS == 1) F[2] = F[2] + A * p;
-  if (AXIS == 2) F[3] = F[3] + A * p;
-  F[4] = F[0] * (T(kGasCp) * Tt + T(0.5) * (u * u + v * v + w * w));
-}
-
-// Wall flux of side `side` (2 * AXIS + 1 on the max side) for a boundary cell
+// Wall flux of side `side` (2 * axis + 1 on the max side) for a boundary cell
 // with state U; `face` indexes the side's inflow table.  Returns false for a
-// zero-flux side (nothing to add).
-template <int AXIS, typename T>
-__device__ __forceinline__ bool wall_flux(const WallBC& bc, int side, int face, const T U[5], T A, T F[5])
+// zero-flux side (nothing to add).  The kinds choose a face state (p, T, u, v, w)
+// and share the flux from it, the tail of CompressibleFarfieldFlux and
+// JetFlux::xWallM (a slip wall has its pressure only).
+template <typename T>
+__device__ __forceinline__ bool wall_flux(const WallBC& bc, int axis, int side, int face, const T U[5], T A, T F[5])
 {
   const int kind = bc.kind[side];
   if (kind == kWallZero) return false;
-  const bool plus = side & 1;
   T p1, T1, u1, v1, w1;
   wall_prim(U, p1, T1, u1, v1, w1);
-  if (kind == kWallSlip) {
-    F[0] = T(0); F[1] = T(0); F[2] = T(0); F[3] = T(0); F[4] = T(0);
-    F[1 + AXIS] = A * p1;
-    return true;
+  T p = p1;
+  F[0] = T(0); F[1] = T(0); F[2] = T(0); F[3] = T(0); F[4] = T(0);
+  if (kind != kWallSlip) {
+    T Tt = T1, u = u1, v = v1, w = w1;
+    if (kind == kWallInflow) {
+      const double* e = bc.table[side] + (size_t)face * 5;
+      if (e[0] == e[0]) p = (T)e[0];               // NaN: pressure of the boundary cell
+      Tt = (T)e[1];
+      u = (T)e[2];
+      v = (T)e[3];
+      w = (T)e[4];
+    } else {
+      // far field: face state from the sign and size of the mean inward Mach number
+      const double* f = bc.ff[side];
+      const T u0 = (T)f[2], v0 = (T)f[3], w0 = (T)f[4], a0 = (T)f[5];
+      const T a1 = dn_sqrt(T(Gas::gamma) * T(Gas::R) * T1);
+      T M0 = (axis == 0 ? u0 : (axis == 1 ? v0 : w0)) / a0;
+      T M1 = (axis == 0 ? u1 : (axis == 1 ? v1 : w1)) / a1;
+      if (side & 1) {
+        M0 = -M0;
+        M1 = -M1;
+      }
+      const T M = T(0.5) * (M0 + M1);
+      // outflow: the reference's test `M <= 1` holds for every M < 0, so the
+      // whole face state comes from the boundary cell
+      if (M >= T(0)) {
+        if (M >= T(1)) p = (T)f[0];                // supersonic, else subsonic inflow
+        Tt = (T)f[1];
+        u = u0;
+        v = v0;
+        w = w0;
+      }
+    }
+    F[0] = A * p / (T(Gas::R) * Tt) * (axis == 0 ? u : (axis == 1 ? v : w));
+    F[1] = F[0] * u;
+    F[2] = F[0] * v;
+    F[3] = F[0] * w;
+    F[4] = F[0] * (T(kGasCp) * Tt + T(0.5) * (u * u + v * v + w * w));
   }
-  if (kind == kWallInflow) {
-    const double* e = bc.table[side] + (size_t)face * 5;
-    const T p = (e[0] == e[0]) ? (T)e[0] : p1;    // NaN: pressure of the boundary cell
-    wall_state_flux<AXIS>(A, p, (T)e[1], (T)e[2], (T)e[3], (T)e[4], F);
-    return true;
-  }
-  // far field: face state from the sign and size of the mean inward Mach number
-  const double* f = bc.ff[side];
-  const T p0 = (T)f[0], T0 = (T)f[1], u0 = (T)f[2], v0 = (T)f[3], w0 = (T)f[4], a0 = (T)f[5];
-  const T a1 = dn_sqrt(T(Gas::gamma) * T(Gas::R) * T1);
-  const T un0 = AXIS == 0 ? u0 : (AXIS == 1 ? v0 : w0);
-  const T un1 = AXIS == 0 ? u1 : (AXIS == 1 ? v1 : w1);
-  const T M0 = plus ? -(un0 / a0) : un0 / a0;
-  const T M1 = plus ? -(un1 / a1) : un1 / a1;
-  const T M = T(0.5) * (M0 + M1);
-  T p, Tt, u, v, w;
-  if (M >= T(0)) {
-    p = M >= T(1) ? p0 : p1;               // supersonic / subsonic inflow
-    Tt = T0; u = u0; v = v0; w = w0;
-  } else {
-    // outflow: the reference's test `M <= 1` holds for every M < 0, so the
-    // whole face state comes from the boundary cell
-    p = p1; Tt = T1; u = u1; v = v1; w = w1;
-  }
-  wall_state_flux<AXIS>(A, p, Tt, u, v, w, F);
+  const T Ap = A * p;
+  F[1] = axis == 0 ? F[1] + Ap : F[1];
+  F[2] = axis == 1 ? F[2] + Ap : F[2];
+  F[3] = axis == 2 ? F[3] + Ap : F[3];
   return true;
 }
 
@@ -117,31 +115,31 @@ __device__ __forceinline__ void add_wall_fluxes(const WallBC& bc, int ni, int nj
 {
   T F[5];
   if (!per_x && ni > 2) {
-    if (i == 0 && wall_flux<0>(bc, 0, j * nk + k, U, Ax, F)) {
+    if (i == 0 && wall_flux(bc, 0, 0, j * nk + k, U, Ax, F)) {
       #pragma unroll
       for (int v = 0; v < 5; ++v) r[v] += F_to_r(v, F[v]);
     }
-    if (i == ni - 1 && wall_flux<0>(bc, 1, j * nk + k, U, Ax, F)) {
+    if (i == ni - 1 && wall_flux(bc, 0, 1, j * nk + k, U, Ax, F)) {
       #pragma unroll
       for (int v = 0; v < 5; ++v) r[v] -= F_to_r(v, F[v]);
     }
   }
   if (!per_y && nj > 2) {
-    if (j == 0 && wall_flux<1>(bc, 2, i * nk + k, U, Ay, F)) {
+    if (j == 0 && wall_flux(bc, 1, 2, i * nk + k, U, Ay, F)) {
       #pragma unroll
       for (int v = 0; v < 5; ++v) r[v] += F_to_r(v, F[v]);
     }
-    if (j == nj - 1 && wall_flux<1>(bc, 3, i * nk + k, U, Ay, F)) {
+    if (j == nj - 1 && wall_flux(bc, 1, 3, i * nk + k, U, Ay, F)) {
       #pragma unroll
       for (int v = 0; v < 5; ++v) r[v] -= F_to_r(v, F[v]);
     }
   }
   if (!per_z && nk > 2) {
-    if (k == 0 && wall_flux<2>(bc, 4, i * nj + j, U, Az, F)) {
+    if (k == 0 && wall_flux(bc, 2, 4, i * nj + j, U, Az, F)) {
       #pragma unroll
       for (int v = 0; v < 5; ++v) r[v] += F_to_r(v, F[v]);
     }
-    if (k == nk - 1 && wall_flux<2>(bc, 5, i * nj + j, U, Az, F)) {
+    if (k == nk - 1 && wall_flux(bc, 2, 5, i * nj + j, U, Az, F)) {
       #pragma unroll
       for (int v = 0; v < 5; ++v) r[v] -= F_to_r(v, F[v]);
     }
