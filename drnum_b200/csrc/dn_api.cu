@@ -3164,13 +3164,13 @@ int dn_autotune(dn_ctx* c, const char* cache_path, double cost_out[DN_NUM_TILE_S
     cudaEventCreate(&e1);
     const bool fp64 = c->precision == DN_FP64;
     // (waves, shortest item): persistent waves for FP32 bulk, or one CTA per
-    // item; 0, 0: FP64 ranges by the cost model.  Of 20 workloads (jet, sphere
+    // item; 0, 0: FP64 ranges by the cost model.  Of 21 workloads (jet, sphere
     // and uneven grids of several scales) the first was the fastest of all
-    // schedules but on two; one CTA per 24 planes took the full-size jet from
+    // schedules but on three; one CTA per 24 planes took the full-size jet from
     // 477 to 454 us a stage, one per 8 planes a grid of few patches from 131 to
-    // 121.
+    // 121, four waves 512 patches from 4147 to 4108.
     const int cand64[3][2] = {{0, 0}, {0, 8}, {0, 16}};
-    const int cand32[5][2] = {{1, 8}, {2, 8}, {0, 8}, {0, 16}, {0, 24}};
+    const int cand32[5][2] = {{1, 8}, {2, 8}, {4, 8}, {0, 8}, {0, 24}};
     const int (*cand)[2] = fp64 ? cand64 : cand32;
     const int n_cand = fp64 ? 3 : 5;
     std::vector<std::vector<int>> shapes(1, c->shape);
