@@ -418,11 +418,11 @@ def run_ours(args, rank, world, local_rank):
     achieved = bytes_per_launch / launch_s / 1e9
     # DRAM traffic of the kernel per launch, from one ncu capture of the three
     # stage launches of a timed RK step on the periodic 192^3 patch
-    # (dram__bytes_read + dram__bytes_write: 36.6, 58.1 and 58.2 B per cell;
+    # (dram__bytes_read + dram__bytes_write: 37.5, 59.5 and 59.7 B per cell;
     # stage 1 reads f(k-1) = f(n) once), averaged and scaled by the cells of
     # this launch: the kernel streams each plane once, so the traffic grows
     # with the cell count
-    TRAFFIC_BYTES_PER_CELL = 50.9
+    TRAFFIC_BYTES_PER_CELL = 52.2
     traffic = TRAFFIC_BYTES_PER_CELL * cells
 
     cpu = None

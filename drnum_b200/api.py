@@ -79,14 +79,14 @@ class AusmPlus(_EulerFlux):
 
 
 class VanLeer(_EulerFlux):
-    """Van Leer flux-vector splitting (fluxes/vanleer.h:29-196), FP64,
-    through the generic functor kernel."""
+    """Van Leer flux-vector splitting (fluxes/vanleer.h:29-196), FP64, a
+    scheme of the specialised fused kernels."""
     scheme = _lib.DN_FLUX_VANLEER
 
 
 class Roe(_EulerFlux):
     """Roe flux with the reference's entropy modification (fluxes/roe.h:
-    29-661), FP64, through the generic functor kernel."""
+    29-661), FP64, a scheme of the specialised fused kernels."""
     scheme = _lib.DN_FLUX_ROE
 
 

@@ -1,6 +1,6 @@
-"""Runs the periodic vortex box through the generic flux-functor stage with
-DrNUM's other Euler fluxes (VanLeer, Roe) and through the specialised AUSM+
-kernel, FP64 on one GPU, and prints each one's throughput.
+"""Runs the periodic vortex box with DrNUM's Euler fluxes (AUSM+, VanLeer,
+Roe) through the specialised stage kernel and with AUSM+ through the generic
+flux-functor stage, FP64 on one GPU, and prints each one's throughput.
 
     python -m drnum_b200.examples.functor_schemes [n] [steps]
 """
@@ -14,7 +14,7 @@ from drnum_b200.api import AusmPlus, B200CartesianIterator, CartesianPatch, Roe,
 def main(n=128, steps=5):
     U0, h, dt = cases.periodic_box(n)
     for name, op in [("AUSM+ (specialised kernel)", AusmPlus()), ("AUSM+ (functor stage)", AusmPlus(functor=True)),
-                     ("VanLeer (functor stage)", VanLeer()), ("Roe (functor stage)", Roe())]:
+                     ("VanLeer (specialised kernel)", VanLeer()), ("Roe (specialised kernel)", Roe())]:
         p = CartesianPatch(n, n, n, spacing=(h, h, h), periodic=(True, True, True))
         p.setField(0, U0)
         it = B200CartesianIterator(op, 0, _lib.DN_FP64)

@@ -1,9 +1,9 @@
-"""The generic flux-functor stage (include/drnum_b200_functor.cuh): the
-built-in VanLeer and Roe schemes bit for bit against the reference's own
-functors (golden fixtures from the compiled reference), AUSM+ through the
-functor kernel bit for bit against the specialised kernel and the
-reference, the patch-face kinds, graph replay, and a caller-written functor
-installed with dn_set_stage_function."""
+"""Flux functors: the built-in VanLeer and Roe schemes (of the specialised
+fused kernels) bit for bit against the reference's own functors (golden
+fixtures from the compiled reference), AUSM+ through the generic functor
+stage (include/drnum_b200_functor.cuh) bit for bit against the specialised
+kernel and the reference, the patch-face kinds, graph replay, and a
+caller-written functor installed with dn_set_stage_function."""
 import ctypes
 import os
 
