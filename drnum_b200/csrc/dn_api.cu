@@ -3168,7 +3168,8 @@ int dn_autotune(dn_ctx* c, const char* cache_path, double cost_out[DN_NUM_TILE_S
     // and uneven grids of several scales) the first was the fastest of all
     // schedules but on three; one CTA per 24 planes took the full-size jet from
     // 477 to 454 us a stage, one per 8 planes a grid of few patches from 131 to
-    // 121, four waves 512 patches from 4147 to 4108.
+    // 121, four waves 512 patches from 4147 to 4108.  One CTA per 16, 32 or 48
+    // planes was fastest on none, nor FP64 ranges of 24, 32 or 48.
     const int cand64[3][2] = {{0, 0}, {0, 8}, {0, 16}};
     const int cand32[5][2] = {{1, 8}, {2, 8}, {4, 8}, {0, 8}, {0, 24}};
     const int (*cand)[2] = fp64 ? cand64 : cand32;

@@ -13,7 +13,7 @@
 // VanLeerFace and RoeFace are schemes of the fused stage kernel
 // (fv_stage.cuh), like AusmPlusFace.  As functors of the generic stage, which
 // reads every cell through the patch view and divides in full, they took
-// 1332 and 1389 us a stage on a periodic 128^3 patch; here 417 and 452 us.
+// 1332 and 1389 us a stage on a periodic 128^3 patch; here 408 and 453 us.
 // AUSM+ also remains a functor of the generic stage
 // (DN_FLUX_AUSMPLUS_FUNCTOR): SchemeFlux<E> combines a functor with the
 // patch-face fluxes of dn_patch_set_bc (far field, slip wall, prescribed

@@ -1,5 +1,6 @@
 // Prints the plane range of a single-patch launch (drnum_b200/csrc/dn_range.h)
-// for each patch "precision ni nj nk" read from standard input.
+// for each patch "precision ni nj nk" read from standard input, and behind it the
+// ranges that the autotuner measures.
 #include <cstdio>
 
 #include "dn_range.h"
@@ -7,7 +8,11 @@
 int main()
 {
   int prec, ni, nj, nk;
-  while (std::scanf("%d %d %d %d", &prec, &ni, &nj, &nk) == 4)
-    std::printf("%d\n", dn::best_ranges(ni, nj, nk, prec == 32 ? 16 : 4, 32, 148,
-                                        prec == 32 ? dn::kRangeFx32 : dn::kRangeF64, 1)[0]);
+  while (std::scanf("%d %d %d %d", &prec, &ni, &nj, &nk) == 4) {
+    const int tj = prec == 32 ? 16 : 4;
+    const dn::RangeCost& c = prec == 32 ? dn::kRangeFx32 : dn::kRangeF64;
+    std::printf("%d", dn::best_ranges(ni, nj, nk, tj, 32, 148, c, 1)[0]);
+    for (int r : dn::best_ranges(ni, nj, nk, tj, 32, 148, c, prec == 32 ? 6 : 4, true)) std::printf(" %d", r);
+    std::printf("\n");
+  }
 }

@@ -40,22 +40,24 @@ def chosen(tmp_path_factory):
     def run(patches):
         text = "\n".join("%d %d %d %d" % (p, *n) for p, n in patches)
         res = subprocess.run([exe], input=text, capture_output=True, text=True, check=True)
-        return [int(x) for x in res.stdout.split()]
+        return [[int(x) for x in line.split()] for line in res.stdout.splitlines()]
     return run
 
 
 def test_choice_against_measured_times(chosen):
     """Within 10 % of the fastest measured range and 1 % (two runs of one side
     differ by up to 0.6 %) of the fixed rule's."""
-    for (prec, n, old, us), ic in zip(MEASURED, chosen([(p, n) for p, n, _, _ in MEASURED])):
+    for (prec, n, old, us), (ic, *_) in zip(MEASURED, chosen([(p, n) for p, n, _, _ in MEASURED])):
         assert ic in us, (prec, n, ic)
         assert us[ic] <= 1.10 * min(us.values()) and us[ic] <= 1.01 * us[old], (prec, n, ic, us)
 
 
 def test_range_bounds(chosen):
-    """Every patch gets a range of at least a plane that its extent and the
+    """Every patch gets ranges of at least a plane that its extent and the
     grid's third extent (65535) allow."""
     patches = [(p, n) for p in (32, 64) for n in [(1, 1, 1), (1, 500, 3), (2, 1, 1), (7, 3, 100000), (100000, 1, 1),
                                                   (300000, 5, 2), (65535, 1, 1), (65536, 4, 32), (40, 2000, 2000)]]
-    for (p, n), ic in zip(patches, chosen(patches)):
-        assert 1 <= ic <= n[0] and -(-n[0] // ic) <= 65535, (p, n, ic)
+    for (p, n), ranges in zip(patches, chosen(patches)):
+        assert 2 <= len(ranges) <= 7 and len(set(ranges[1:])) == len(ranges) - 1, (p, n, ranges)
+        for ic in ranges:
+            assert 1 <= ic <= n[0] and -(-n[0] // ic) <= 65535, (p, n, ranges)
